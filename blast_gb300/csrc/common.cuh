@@ -55,11 +55,32 @@ int launch_syrk_lower(int m, int k, int trans_a, double alpha, const double* A, 
                       double beta, const double* C, int ldc, int64_t sc, double* D, int ldd, int64_t sd,
                       int64_t batch, cudaStream_t s);
 
-// Uniform batch of Cholesky solves (or factorisations: nrhs = 0; or solves with a given factor:
-// A = nullptr) on the CTA-per-matrix kernels of posv_cta.cu, n <= 512. L may equal A, X may equal B.
-int launch_posv_cta_strided(int n, int nrhs, const double* A, int lda, int64_t sa, double* L, int ldl,
-                            int64_t sl, const double* B, int ldb, int64_t sb, double* X, int ldx, int64_t sx,
-                            int32_t* info, int64_t batch, cudaStream_t s);
+// Uniform batch of solves with given Cholesky factors on the CTA-per-matrix kernel of posv_cta.cu, n <= 512. X
+// may equal B.
+int launch_potrs_cta_strided(int n, int nrhs, double* L, int ldl, int64_t sl, const double* B, int ldb, int64_t sb,
+                             double* X, int ldx, int64_t sx, int64_t batch, cudaStream_t s);
+
+// Square matrices with n > kFixMinN - 1 are factored in 64-bit fixed point (potrf_fix.cu); up to 16 rows the
+// whole matrix is one panel of it, and the kernels that run a matrix in a thread, a quad or a warp
+// keep the products in binary64.
+constexpr int kFixMinN = 17;
+// L := chol(A), uniform batch, n <= 512. W: 8 bytes per entry of scratch with leading dimension ldw (nullptr: L
+// itself); L2: a second copy of the factor (nullptr: none). L may equal A, L2 may equal W.
+int launch_potrf_fix(int n, const double* A, int lda, int64_t sa, double* L, int ldl, int64_t sl, double* W, int ldw,
+                     int64_t sw, double* L2, int ldl2, int64_t sl2, int32_t* info, int64_t batch, cudaStream_t s);
+// Ragged: the instances with A and at least min_n rows; info is written for these only.
+int launch_potrf_fix(const blastgpu_posv_desc* desc, int min_n, int max_n, int32_t* info, int64_t batch, cudaStream_t s);
+int launch_potrf_fix(const blastgpu_posv_bwd_desc* desc, int min_n, int max_n, int32_t* info, int64_t batch,
+                     cudaStream_t s);
+
+// Factorisation and, with nrhs > 0, solve in fixed point, two matrices per warp (posv_pair.cu), n <= 64. L may
+// equal A, X may equal B.
+constexpr int kPairMaxN = 64;
+int launch_posv_pair(int n, int nrhs, const double* A, int lda, int64_t sa, double* L, int ldl, int64_t sl,
+                     const double* B, int ldb, int64_t sb, double* X, int ldx, int64_t sx, int32_t* info, int64_t batch,
+                     cudaStream_t s);
+// Ragged: the instances with A and min_n <= rows <= max_n.
+int launch_posv_pair(const blastgpu_posv_desc* desc, int min_n, int max_n, int32_t* info, int64_t batch, cudaStream_t s);
 
 // Ragged binary64 Cholesky solves with every n <= 128 on the warp-per-matrix kernel of
 // posv_warp.cu (descriptors as for blastgpu_dposv_batched).

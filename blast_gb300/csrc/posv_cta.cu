@@ -890,22 +890,14 @@ struct CtaArgs {
     int max_iter;
 };
 
-// Plain binary64 path: factor into L, then X = A^{-1} B column by column.
+// Binary64 solves with the factor in L: X = A^{-1} B column by column.
 template <int MAXR, class Batch>
-__global__ void __launch_bounds__(kThreads, MAXR <= 8 ? 2 : 1) posv_cta_f64_kernel(Batch batch, CtaArgs args) {
-    using S = Smem<double, MAXR>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* buf = reinterpret_cast<double*>(smem_raw);
-    double* vec = buf + S::kBufElems;
-    __shared__ int s_info;
+__global__ void __launch_bounds__(kThreads, 2) potrs_cta_kernel(Batch batch, CtaArgs args) {
+    __shared__ double vec[32 * MAXR];
     int64_t const b = blockIdx.x;
     if (b >= args.batch) return;
     CtaItem const it = batch.get(b);
     int const n = it.n;
-    if (it.A != nullptr) {  // A == nullptr: solves with the given factor L only
-        int const info = cta_potrf<double, MAXR>(n, it.A, it.lda, it.L, it.ldl, buf, &s_info);
-        if (threadIdx.x == 0 && args.info) args.info[b] = info;
-    }
     for (int c = 0; c < it.nrhs; ++c) {
         for (int i = threadIdx.x; i < n; i += kThreads) vec[i] = it.B[i + (int64_t)c * it.ldb];
         __syncthreads();
@@ -1051,27 +1043,16 @@ struct DescBwd {
     }
 };
 
+// The factor is in L. info (nullptr if the factorisation wrote it): set to 0.
 template <int MAXR, class Batch>
-// Two CTAs per SM up to n = 128 (MAXR <= 4 fits 128 registers per thread); larger bins keep the
-// register budget of one CTA per SM.
-__global__ void __launch_bounds__(kThreads, MAXR <= 4 ? 2 : 1)
-    posv_bwd_kernel(Batch batch, int64_t count, int recompute, int32_t* info) {
-    using S = Smem<double, MAXR>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* buf = reinterpret_cast<double*>(smem_raw);
-    double* vec = buf + S::kBufElems;
-    __shared__ int s_info;
+__global__ void __launch_bounds__(kThreads, 2) posv_bwd_kernel(Batch batch, int64_t count, int32_t* info) {
+    constexpr int NMAX = 32 * MAXR;
+    __shared__ double vec[2 * NMAX];
     int64_t const b = blockIdx.x;
     if (b >= count) return;
     BwdItem const it = batch.get(b);
     int const n = it.n, tid = threadIdx.x;
-    if (recompute) {
-        int const r = cta_potrf<double, MAXR>(n, it.A, it.lda, it.L, it.ldl, buf, &s_info);
-        if (tid == 0 && info) info[b] = r;
-    } else if (tid == 0 && info) {
-        info[b] = 0;
-    }
-    __syncthreads();
+    if (tid == 0 && info) info[b] = 0;
     for (int c = 0; c < it.nrhs; ++c) {
         for (int i = tid; i < n; i += kThreads) vec[i] = it.G[i + (int64_t)c * it.ldg];
         __syncthreads();
@@ -1083,7 +1064,7 @@ __global__ void __launch_bounds__(kThreads, MAXR <= 4 ? 2 : 1)
     // right-hand side, GB (still in vec) and X come from shared memory.
     int const lane = tid & 31, warp = tid >> 5;
     if (it.nrhs == 1) {
-        double* xs = vec + S::NMAX;
+        double* xs = vec + NMAX;
         for (int i = tid; i < n; i += kThreads) xs[i] = it.X[i];
         __syncthreads();
         for (int j = warp; j < n; j += kWarps) {
@@ -1105,11 +1086,8 @@ __global__ void __launch_bounds__(kThreads, MAXR <= 4 ? 2 : 1)
 }
 
 template <int MAXR>
-int launch_bwd(DescBwd const& batch, int64_t count, int recompute, int32_t* info, cudaStream_t s) {
-    size_t const smem = Smem<double, MAXR>::kBytes;
-    cudaError_t e = ensure_smem<posv_bwd_kernel<MAXR, DescBwd>>(smem);
-    if (e != cudaSuccess) { set_cuda_error(e); return BLASTGPU_ERR_CUDA; }
-    posv_bwd_kernel<MAXR, DescBwd><<<(unsigned)count, kThreads, smem, s>>>(batch, count, recompute, info);
+int launch_bwd(DescBwd const& batch, int64_t count, int32_t* info, cudaStream_t s) {
+    posv_bwd_kernel<MAXR, DescBwd><<<(unsigned)count, kThreads, 0, s>>>(batch, count, info);
     return check_launch();
 }
 
@@ -1126,7 +1104,6 @@ cudaError_t launch_mixed(Batch const& batch, CtaArgs const& args, cudaStream_t s
 // default 0, the fastest measured on GB300).
 template <int MAXR, class Batch>
 int launch_cta(bool mixed, Batch const& batch, CtaArgs const& args, cudaStream_t s) {
-    size_t const smem = Smem<double, MAXR>::kBytes;
     cudaError_t e = cudaSuccess;
     if (mixed) {
         // only descriptor batches carry the mixed path's workspace offsets
@@ -1141,8 +1118,7 @@ int launch_cta(bool mixed, Batch const& batch, CtaArgs const& args, cudaStream_t
             return BLASTGPU_ERR_NOT_IMPLEMENTED;
         }
     } else {
-        e = ensure_smem<posv_cta_f64_kernel<MAXR, Batch>>(smem);
-        if (e == cudaSuccess) posv_cta_f64_kernel<MAXR, Batch><<<(unsigned)args.batch, kThreads, smem, s>>>(batch, args);
+        potrs_cta_kernel<MAXR, Batch><<<(unsigned)args.batch, kThreads, 0, s>>>(batch, args);
     }
     if (e != cudaSuccess) { set_cuda_error(e); return BLASTGPU_ERR_CUDA; }
     return check_launch();
@@ -1161,11 +1137,10 @@ int dispatch_cta(bool mixed, int max_n, Batch const& batch, CtaArgs const& args,
 
 }  // namespace
 
-int launch_posv_cta_strided(int n, int nrhs, const double* A, int lda, int64_t sa, double* L, int ldl,
-                            int64_t sl, const double* B, int ldb, int64_t sb, double* X, int ldx, int64_t sx,
-                            int32_t* info, int64_t batch, cudaStream_t s) {
-    StridedPosv const p{n, nrhs, A, lda, sa, L, ldl, sl, B, ldb, sb, X, ldx, sx};
-    CtaArgs const a{batch, info, nullptr, nullptr, 0.0, 0};
+int launch_potrs_cta_strided(int n, int nrhs, double* L, int ldl, int64_t sl, const double* B, int ldb, int64_t sb,
+                             double* X, int ldx, int64_t sx, int64_t batch, cudaStream_t s) {
+    StridedPosv const p{n, nrhs, nullptr, 1, 0, L, ldl, sl, B, ldb, sb, X, ldx, sx};
+    CtaArgs const a{batch, nullptr, nullptr, nullptr, 0.0, 0};
     return dispatch_cta(false, n, p, a, s);
 }
 
@@ -1239,7 +1214,9 @@ int blastgpu_dposv_batched(const blastgpu_posv_desc* desc, int64_t batch, int ma
     // "posv.warp.n<bin>" (default 1): batches with every n <= 128 on the warp-per-matrix kernel
     if (max_n <= 128 && tune_get_bin("posv.warp", max_n, 1) != 0)
         return launch_posv_warp(desc, batch, max_n, info, as_cuda(stream));
-    CtaArgs a{batch, info, nullptr, nullptr, 0.0, 0};
+    int const st = launch_potrf_fix(desc, 0, max_n, info, batch, as_cuda(stream));
+    if (st != BLASTGPU_SUCCESS) return st;
+    CtaArgs a{batch, nullptr, nullptr, nullptr, 0.0, 0};
     return dispatch_cta(false, max_n, DescPosv{desc, nullptr}, a, as_cuda(stream));
 }
 
@@ -1271,11 +1248,16 @@ int blastgpu_dposv_bwd_batched(const blastgpu_posv_bwd_desc* desc, int64_t batch
     // "posv.warp_bwd.n<bin>" (default 1): batches with every n <= 128 one warp per matrix
     if (max_n <= 128 && tune_get_bin("posv.warp_bwd", max_n, 1) != 0)
         return launch_posv_bwd_warp(desc, batch, max_n, recompute, info, s);
-    if (max_n <= 64) return launch_bwd<2>(d, batch, recompute, info, s);
-    if (max_n <= 128) return launch_bwd<4>(d, batch, recompute, info, s);
-    if (max_n <= 256) return launch_bwd<8>(d, batch, recompute, info, s);
-    if (max_n <= 512) return launch_bwd<16>(d, batch, recompute, info, s);
-    return BLASTGPU_ERR_TOO_LARGE;
+    if (max_n > 512) return BLASTGPU_ERR_TOO_LARGE;
+    if (recompute) {
+        int const st = launch_potrf_fix(desc, 0, max_n, info, batch, s);
+        if (st != BLASTGPU_SUCCESS) return st;
+        info = nullptr;
+    }
+    if (max_n <= 64) return launch_bwd<2>(d, batch, info, s);
+    if (max_n <= 128) return launch_bwd<4>(d, batch, info, s);
+    if (max_n <= 256) return launch_bwd<8>(d, batch, info, s);
+    return launch_bwd<16>(d, batch, info, s);
 }
 
 }  // extern "C"

@@ -1,20 +1,16 @@
-// Ragged Cholesky solves for small n (n <= 128), binary64: one warp per matrix.
+// Ragged Cholesky solves for small n (n <= 128), binary64: one warp per matrix. Matrices of kFixMinN
+// rows and more arrive factored (potrf_fix.cu); smaller ones are factored here.
 //
 // Reference: blast::potrf (dense/Potrf.hpp:66-106), left-looking in strips of 4 columns: each
 // element of a strip first takes the fused products of all earlier columns in ascending order
 // (the ger(-1, ...) loop), then RegisterMatrix::potrf / ::trsm (RegisterMatrix.hpp:566-602,
 // 710-739) finish the strip column by column. The solves follow dense/Trsm.hpp:39-65.
 //
-// Mapping: lane l owns rows l, l + 32, ... of its matrix (MAXT row blocks), so each strip's
-// register tile is MAXT x 4 per lane, the earlier columns are read coalesced (a warp reads 32
-// consecutive rows of a column), and the strip's own rows are broadcast loads. The diagonal 4 x 4
-// block lives in 4 consecutive lanes; its entries reach the other lanes by shuffles. Every element
-// sees the same fused multiply-adds, in the same order, as the thread-per-matrix kernel
-// (potrf_tile: the products of column l before those of column l + 1; then, for column c of the
-// strip, the terms of the strip's columns j < c, and the scaling by the reciprocal square root of
-// the pivot), so the factor and the solutions are the same bits. A thread per matrix needs far
-// more matrices than a ragged batch of small n has to fill the chip, and a CTA per matrix spends
-// its time on barriers; a warp per matrix has neither problem.
+// Mapping: lane l owns rows l, l + 32, ... of its matrix (MAXT row blocks). Every element sees the
+// same fused multiply-adds, in the same order, as the thread-per-matrix kernel, so the factor and
+// the solutions are the same bits. A thread per matrix needs far more matrices than a ragged batch
+// of small n has to fill the chip, and a CTA per matrix spends its time on barriers; a warp per
+// matrix has neither problem.
 //
 // Solves, one right-hand side at a time: the forward substitution is a column sweep (once x_l is
 // final, every row below takes its term), which keeps each row's ascending order. The backward
@@ -29,105 +25,51 @@ namespace {
 
 constexpr int kWarpsPerCta = 4;
 
-// Column C of the strip at k: the terms of the strip's columns j < C (their final, scaled
-// values), then the scaling by y = rsqrt_nr(pivot). The strip's rows k .. k+3 are in block T0;
-// blocks above it hold no rows at or below k and are left out at compile time, rows above k + C
-// in block T0 by a predicate.
-template <int MAXT, int T0, int C>
-__device__ __forceinline__ void strip_column(double (&acc)[MAXT][4], int k, int n, int lane, int& info) {
-    int const owner = (k + C) & 31;
+// Column C of the strip at k of a matrix with at most 32 rows, lane = row: the terms of the strip's columns
+// j < C (their final, scaled values), then the scaling by y = rsqrt_nr(pivot).
+template <int C>
+__device__ __forceinline__ void strip_column(double (&acc)[4], int k, int n, int lane, int& info) {
+    int const owner = k + C;
+    bool const mine = lane - k >= C && lane < n;
 #pragma unroll
     for (int j = 0; j < C; ++j) {
         // l_{k+C, k+j}: row k + C's final value in column j, from the lane that holds it
-        double const lcj = __shfl_sync(0xffffffffu, acc[T0][j], owner);
-#pragma unroll
-        for (int t = T0; t < MAXT; ++t) {
-            int const i = lane + 32 * t;
-            if (i - k >= C && i < n) acc[t][C] = fma(-lcj, acc[t][j], acc[t][C]);
-        }
+        double const lcj = __shfl_sync(0xffffffffu, acc[j], owner);
+        if (mine) acc[C] = fma(-lcj, acc[j], acc[C]);
     }
-    double const s = __shfl_sync(0xffffffffu, acc[T0][C], owner);
+    double const s = __shfl_sync(0xffffffffu, acc[C], owner);
     if (!(s > 0.0) && info == 0) info = k + C + 1;
     double const y = rsqrt_nr(s);
-#pragma unroll
-    for (int t = T0; t < MAXT; ++t) {
-        int const i = lane + 32 * t;
-        if (i - k >= C && i < n) acc[t][C] *= y;
-    }
-}
-
-// One strip (columns k .. k+nc-1) of the left-looking Cholesky, its rows in blocks T0 .. MAXT-1.
-template <int MAXT, int T0>
-__device__ __forceinline__ void warp_strip(int n, int k, const double* A, int lda, double* L, int ldl, int lane,
-                                           int& info) {
-    int const nc = min(4, n - k);
-    double acc[MAXT][4];
-#pragma unroll
-    for (int t = T0; t < MAXT; ++t)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            int const i = lane + 32 * t;
-            acc[t][c] = (c < nc && i < n && i - k >= c) ? A[i + (int64_t)(k + c) * lda] : 0.0;
-        }
-    // the earlier columns in ascending order, the next column's loads issued first
-    if (k > 0) {
-        double a[MAXT], b[4];
-#pragma unroll
-        for (int t = T0; t < MAXT; ++t) {
-            int const i = lane + 32 * t;
-            a[t] = (i < n && i >= k) ? L[i] : 0.0;
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) b[c] = c < nc ? L[k + c] : 0.0;
-        for (int l = 0; l < k; ++l) {
-            double an[MAXT], bn[4];
-            int const ln = l + 1 < k ? l + 1 : l;
-            double const* col = L + (int64_t)ln * ldl;
-#pragma unroll
-            for (int t = T0; t < MAXT; ++t) {
-                int const i = lane + 32 * t;
-                an[t] = (i < n && i >= k) ? col[i] : 0.0;
-            }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) bn[c] = c < nc ? col[k + c] : 0.0;
-#pragma unroll
-            for (int t = T0; t < MAXT; ++t) {
-                int const i = lane + 32 * t;
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (t > T0 || i - k >= c) acc[t][c] = fma(-a[t], b[c], acc[t][c]);
-            }
-#pragma unroll
-            for (int t = T0; t < MAXT; ++t) a[t] = an[t];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = bn[c];
-        }
-    }
-    strip_column<MAXT, T0, 0>(acc, k, n, lane, info);
-    if (nc > 1) strip_column<MAXT, T0, 1>(acc, k, n, lane, info);
-    if (nc > 2) strip_column<MAXT, T0, 2>(acc, k, n, lane, info);
-    if (nc > 3) strip_column<MAXT, T0, 3>(acc, k, n, lane, info);
-#pragma unroll
-    for (int t = T0; t < MAXT; ++t)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            int const i = lane + 32 * t;
-            if (c < nc && i < n && i - k >= c) L[i + (int64_t)(k + c) * ldl] = acc[t][c];
-        }
+    if (mine) acc[C] *= y;
 }
 
 // Left-looking Cholesky of the n x n matrix A (lower triangle read) into L (lower triangle
-// written), one warp. Returns 0 or the first bad pivot + 1, the same in every lane.
-template <int MAXT>
+// written), n < kFixMinN, one warp. Returns 0 or the first bad pivot + 1, the same in every lane.
 __device__ int warp_potrf(int n, const double* A, int lda, double* L, int ldl, int lane) {
     int info = 0;
     for (int k = 0; k < n; k += 4) {
-        switch (k >> 5) {  // the block holding rows k .. k+3 (k is a multiple of 4)
-            case 0: warp_strip<MAXT, 0>(n, k, A, lda, L, ldl, lane, info); break;
-            case 1: if constexpr (MAXT > 1) warp_strip<MAXT, (MAXT > 1 ? 1 : 0)>(n, k, A, lda, L, ldl, lane, info); break;
-            case 2: if constexpr (MAXT > 2) warp_strip<MAXT, (MAXT > 2 ? 2 : 0)>(n, k, A, lda, L, ldl, lane, info); break;
-            default: if constexpr (MAXT > 3) warp_strip<MAXT, (MAXT > 3 ? 3 : 0)>(n, k, A, lda, L, ldl, lane, info); break;
+        int const nc = min(4, n - k);
+        bool const below = lane < n && lane >= k;
+        double acc[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] = (c < nc && lane < n && lane - k >= c) ? A[lane + (int64_t)(k + c) * lda] : 0.0;
+        // the earlier columns in ascending order
+        for (int l = 0; l < k; ++l) {
+            double const* col = L + (int64_t)l * ldl;
+            double const a = below ? col[lane] : 0.0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                double const b = c < nc ? col[k + c] : 0.0;
+                if (lane - k >= c) acc[c] = fma(-a, b, acc[c]);
+            }
         }
+        strip_column<0>(acc, k, n, lane, info);
+        if (nc > 1) strip_column<1>(acc, k, n, lane, info);
+        if (nc > 2) strip_column<2>(acc, k, n, lane, info);
+        if (nc > 3) strip_column<3>(acc, k, n, lane, info);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (c < nc && lane < n && lane - k >= c) L[lane + (int64_t)(k + c) * ldl] = acc[c];
         __syncwarp();  // the strip's columns are read by every lane from the next strip on
     }
     return info;
@@ -223,8 +165,8 @@ __device__ void warp_potrs_column(int n, const double* L, int ldl, const double*
 // blocks past its last row cost nothing.
 template <int NB>
 __device__ __forceinline__ void warp_posv(blastgpu_posv_desc const& dsc, int n, double* xs, int lane, int32_t* info_b) {
-    if (dsc.A.data != nullptr) {  // A == nullptr: solves with the given factor L only
-        int const r = warp_potrf<NB>(n, dsc.A.data, dsc.A.ld, dsc.L.data, dsc.L.ld, lane);
+    if (NB == 1 && dsc.A.data != nullptr && n < kFixMinN) {  // else the factor is in L
+        int const r = warp_potrf(n, dsc.A.data, dsc.A.ld, dsc.L.data, dsc.L.ld, lane);
         if (info_b && lane == 0) *info_b = r;
     }
     for (int j = 0; j < dsc.B.cols; ++j)
@@ -234,7 +176,7 @@ __device__ __forceinline__ void warp_posv(blastgpu_posv_desc const& dsc, int n, 
 
 template <int MAXT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) posv_warp_kernel(const blastgpu_posv_desc* desc, int64_t count,
-                                                                     int32_t* info) {
+                                                                     bool paired, int32_t* info) {
     __shared__ double xs_all[kWarpsPerCta][32 * MAXT];
     int const w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int64_t const b = (int64_t)blockIdx.x * kWarpsPerCta + w;
@@ -242,6 +184,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) posv_warp_kernel(const blas
     blastgpu_posv_desc const& dsc = desc[b];
     int const n = dsc.A.rows;
     if (n > 32 * MAXT) return;  // the launch's max_n bounds every instance
+    if (paired && n >= kFixMinN && dsc.A.data != nullptr) return;  // solved by posv_pair.cu
     int32_t* const info_b = info ? info + b : nullptr;
     switch ((n + 31) >> 5) {
         case 0:
@@ -258,10 +201,10 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) posv_warp_kernel(const blas
 template <int NB>
 __device__ __forceinline__ void warp_posv_bwd(blastgpu_posv_bwd_desc const& d, int n, int recompute, double* xs,
                                               int lane, int32_t* info_b) {
-    if (recompute) {
-        int const r = warp_potrf<NB>(n, d.A.data, d.A.ld, d.L.data, d.L.ld, lane);
+    if (NB == 1 && recompute && n < kFixMinN) {  // else the factor is in L
+        int const r = warp_potrf(n, d.A.data, d.A.ld, d.L.data, d.L.ld, lane);
         if (info_b && lane == 0) *info_b = r;
-    } else if (info_b && lane == 0) {
+    } else if (!recompute && info_b && lane == 0) {
         *info_b = 0;
     }
     int const nrhs = d.X.cols;
@@ -328,6 +271,10 @@ int launch_posv_bwd_warp(const blastgpu_posv_bwd_desc* desc, int64_t count, int 
     if (count == 0) return BLASTGPU_SUCCESS;
     int64_t const blocks = (count + kWarpsPerCta - 1) / kWarpsPerCta;
     if (blocks > 0x7fffffff) return BLASTGPU_ERR_TOO_LARGE;
+    if (recompute && max_n >= kFixMinN) {
+        int const st = launch_potrf_fix(desc, kFixMinN, max_n, info, count, s);
+        if (st != BLASTGPU_SUCCESS) return st;
+    }
     unsigned const g = (unsigned)blocks, t = kWarpsPerCta * 32;
     if (max_n <= 32) posv_bwd_warp_kernel<1><<<g, t, 0, s>>>(desc, count, recompute, info);
     else if (max_n <= 64) posv_bwd_warp_kernel<2><<<g, t, 0, s>>>(desc, count, recompute, info);
@@ -342,10 +289,16 @@ int launch_posv_warp(const blastgpu_posv_desc* desc, int64_t count, int max_n, i
     if (count == 0) return BLASTGPU_SUCCESS;
     int64_t const blocks = (count + kWarpsPerCta - 1) / kWarpsPerCta;
     if (blocks > 0x7fffffff) return BLASTGPU_ERR_TOO_LARGE;
+    bool const paired = max_n <= kPairMaxN;
+    if (max_n >= kFixMinN) {
+        int const st = paired ? launch_posv_pair(desc, kFixMinN, max_n, info, count, s)
+                              : launch_potrf_fix(desc, kFixMinN, max_n, info, count, s);
+        if (st != BLASTGPU_SUCCESS) return st;
+    }
     unsigned const g = (unsigned)blocks, t = kWarpsPerCta * 32;
-    if (max_n <= 32) posv_warp_kernel<1><<<g, t, 0, s>>>(desc, count, info);
-    else if (max_n <= 64) posv_warp_kernel<2><<<g, t, 0, s>>>(desc, count, info);
-    else if (max_n <= 128) posv_warp_kernel<4><<<g, t, 0, s>>>(desc, count, info);
+    if (max_n <= 32) posv_warp_kernel<1><<<g, t, 0, s>>>(desc, count, paired, info);
+    else if (max_n <= 64) posv_warp_kernel<2><<<g, t, 0, s>>>(desc, count, paired, info);
+    else if (max_n <= 128) posv_warp_kernel<4><<<g, t, 0, s>>>(desc, count, paired, info);
     else return BLASTGPU_ERR_TOO_LARGE;
     return check_launch();
 }

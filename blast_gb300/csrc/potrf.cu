@@ -56,46 +56,6 @@ struct LoadSrc {
     }
 };
 
-// SyrkSrc: beta*C + alpha*A*A^T (A: n x K, or K x n read transposed), formed tile by tile in the
-// order of blast::syrkLower (dense/Syrk.hpp:15-145): v = beta*c_ij rounded (RegisterMatrix::load(
-// beta, ..)), then for l ascending v = fma(alpha*a_il, a_jl, v) (RegisterMatrix::ger(alpha, ..)).
-// The factorisation then runs on exactly the values syrkLower would have stored. ALPHA1: alpha is
-// 1, so alpha*a_il is a_il exactly and its multiplication is left out.
-template <bool ALPHA1>
-struct SyrkSrc {
-    const double* A;
-    int64_t lda;
-    int K;
-    bool trans;
-    double alpha, beta;
-    const double* C;
-    int64_t ldc;
-    __device__ __forceinline__ double a(int i, int l) const {
-        return trans ? A[l + (int64_t)i * lda] : A[i + (int64_t)l * lda];
-    }
-    template <int KM, int KN, bool DIAG>
-    __device__ __forceinline__ void fill(double (&acc)[KM][KN], int n, int k, int i, int nc) const {
-#pragma unroll
-        for (int c = 0; c < KN; ++c)
-#pragma unroll
-            for (int r = 0; r < KM; ++r)
-                acc[r][c] = (c < nc && i + r < n && (!DIAG || r >= c)) ? beta * C[(i + r) + (int64_t)(k + c) * ldc]
-                                                                      : 0.0;
-        for (int l = 0; l < K; ++l) {
-            double ax[KM], b[KN];
-#pragma unroll
-            for (int r = 0; r < KM; ++r) ax[r] = (i + r < n) ? (ALPHA1 ? a(i + r, l) : alpha * a(i + r, l)) : 0.0;
-#pragma unroll
-            for (int c = 0; c < KN; ++c) b[c] = (c < nc) ? a(k + c, l) : 0.0;
-#pragma unroll
-            for (int c = 0; c < KN; ++c)
-#pragma unroll
-                for (int r = 0; r < KM; ++r)
-                    if (!DIAG || r >= c) acc[r][c] = fma(ax[r], b[c], acc[r][c]);
-        }
-    }
-};
-
 // One KM x KN register tile of the left-looking strip k (rows i .. i+KM-1 of the n rows passed
 // as the first argument, the matrix's row count). DIAG: the strip's
 // first tile, which holds the diagonal block; its strictly upper entries (r < c) are never stored,
@@ -641,6 +601,8 @@ struct MirrorHook {
     }
 };
 
+// FACTOR false: the factor is in p.L (potrf_fix.cu left it there and in host memory); solves only.
+template <bool FACTOR>
 __global__ void __launch_bounds__(32, 12) posv_mirror_kernel(PosvArgs p, MirrorOut o) {
     int64_t const b0 = (int64_t)blockIdx.x * 32;
     int const lane = threadIdx.x;
@@ -650,10 +612,12 @@ __global__ void __launch_bounds__(32, 12) posv_mirror_kernel(PosvArgs p, MirrorO
     int const cnt = full ? 32 : (int)(p.batch - b0);
     if (full) {  // A arrives and L leaves strip by strip, in whole-warp copies
         double* L = p.L + b * p.sl;
-        MirrorHook const hook{n,     lane,  p.A + b0 * p.sa,  p.lda,  p.sa,  p.L + b0 * p.sl,
-                              p.ldl, p.sl,  o.Lh + b0 * o.slh, o.ldlh, o.slh};
-        int const info = potrf_thread_src<4, 4>(n, LoadSrc<ColAddr>{L, ColAddr{p.ldl}}, L, ColAddr{p.ldl}, hook);
-        if (p.info) p.info[b] = info;
+        if constexpr (FACTOR) {
+            MirrorHook const hook{n,     lane,  p.A + b0 * p.sa,  p.lda,  p.sa,  p.L + b0 * p.sl,
+                                  p.ldl, p.sl,  o.Lh + b0 * o.slh, o.ldlh, o.slh};
+            int const info = potrf_thread_src<4, 4>(n, LoadSrc<ColAddr>{L, ColAddr{p.ldl}}, L, ColAddr{p.ldl}, hook);
+            if (p.info) p.info[b] = info;
+        }
         if (p.nrhs > 0) {  // B staged into the working copy of X, then solved in place
             __syncwarp();
             for (int j0 = 0; j0 < p.nrhs; j0 += 4)
@@ -666,8 +630,10 @@ __global__ void __launch_bounds__(32, 12) posv_mirror_kernel(PosvArgs p, MirrorO
         }
     } else if (b < p.batch) {
         double* L = p.L + b * p.sl;
-        int const info = potrf_thread<4, 4>(n, p.A + b * p.sa, ColAddr{p.lda}, L, ColAddr{p.ldl});
-        if (p.info) p.info[b] = info;
+        if constexpr (FACTOR) {
+            int const info = potrf_thread<4, 4>(n, p.A + b * p.sa, ColAddr{p.lda}, L, ColAddr{p.ldl});
+            if (p.info) p.info[b] = info;
+        }
         if (p.nrhs > 0) {
             double* X = p.X + b * p.sx;
             trsm_lower_thread(n, p.nrhs, L, p.ldl, p.B + b * p.sb, p.ldb, X, p.ldx);
@@ -675,7 +641,7 @@ __global__ void __launch_bounds__(32, 12) posv_mirror_kernel(PosvArgs p, MirrorO
         }
     }
     __syncwarp();
-    if (!full)
+    if (FACTOR && !full)
         warp_copy_cols(n, 0, n, true, cnt, p.L + b0 * p.sl, p.ldl, p.sl, o.Lh + b0 * o.slh, o.ldlh, o.slh, lane);
     if (p.nrhs > 0)
         warp_copy_cols(n, 0, p.nrhs, false, cnt, p.X + b0 * p.sx, p.ldx, p.sx, o.Xh + b0 * o.sxh, o.ldxh, o.sxh, lane);
@@ -701,27 +667,6 @@ __global__ void __launch_bounds__(32, 12) potrf_desc_kernel(const blastgpu_potrf
     if (info) info[b] = r;
 }
 
-// D = chol(beta*C + alpha*op(A)*op(A)^T), lower, one thread per instance: syrkLower's values are
-// formed inside the factorisation's register tiles and never stored.
-struct SyrkPotrfArgs {
-    int n, k, trans;
-    double alpha, beta;
-    const double* A; int lda; int64_t sa;
-    const double* C; int ldc; int64_t sc;
-    double* D; int ldd; int64_t sd;
-    int32_t* info;
-    int64_t batch;
-};
-
-template <bool ALPHA1>
-__global__ void __launch_bounds__(32, 12) syrk_potrf_thread_kernel(SyrkPotrfArgs p) {
-    int64_t const b = (int64_t)blockIdx.x * 32 + threadIdx.x;
-    if (b >= p.batch) return;
-    SyrkSrc<ALPHA1> const src{p.A + b * p.sa, p.lda, p.k, p.trans != 0, p.alpha, p.beta, p.C + b * p.sc, p.ldc};
-    int const info = potrf_thread_src<4, 4>(p.n, src, p.D + b * p.sd, ColAddr{p.ldd});
-    if (p.info) p.info[b] = info;
-}
-
 // Quads ("posv.quad.n<bin>" = T) when the batch holds fewer than T / 100 full warps per SM
 // sub-partition. Defaults from measurements on GB300 (n = 16: quads win at 8,000 matrices and lose
 // at 16,000; n = 32, 48 and 64: they win up to 24,000 and lose at 50,000; n = 96 and 128: 3.3-3.7x
@@ -745,13 +690,23 @@ int launch_posv(PosvArgs const& p, cudaStream_t stream) {
         }
         return BLASTGPU_SUCCESS;
     }
-    // Square matrices from "posv.cta_min_n" (default 65) on go to the CTA-per-matrix kernels: one
-    // thread per matrix would need more registers than a thread has, and a batch of them leaves
-    // most of the chip idle.
-    if ((p.m == 0 || p.m == p.n) && p.n >= tune_get("posv.cta_min_n", 65) && p.n <= 512)
-        return launch_posv_cta_strided(p.n, p.nrhs, p.mode == 2 ? nullptr : p.A, p.lda, p.sa, p.L, p.ldl, p.sl,
-                                       p.B, p.ldb, p.sb, p.X, p.ldx, p.sx, p.mode == 2 ? nullptr : p.info,
-                                       p.batch, stream);
+    // Square matrices of kFixMinN rows and more are factored in fixed point; the solves follow.
+    if ((p.m == 0 || p.m == p.n) && p.mode != 2 && p.n >= kFixMinN && p.n <= 512) {
+        if (p.n <= kPairMaxN)
+            return launch_posv_pair(p.n, p.mode == 1 ? p.nrhs : 0, p.A, p.lda, p.sa, p.L, p.ldl, p.sl, p.B, p.ldb, p.sb,
+                                    p.X, p.ldx, p.sx, p.info, p.batch, stream);
+        int const st = launch_potrf_fix(p.n, p.A, p.lda, p.sa, p.L, p.ldl, p.sl, nullptr, 0, 0, nullptr, 0, 0, p.info,
+                                        p.batch, stream);
+        if (st != BLASTGPU_SUCCESS || p.mode == 0 || p.nrhs == 0) return st;
+        PosvArgs q = p;
+        q.mode = 2;
+        return launch_posv(q, stream);
+    }
+    // Solves from "posv.cta_min_n" (default 65) on go to the CTA-per-matrix kernel: a batch of one
+    // thread per matrix leaves most of the chip idle.
+    if (p.mode == 2 && p.n >= tune_get("posv.cta_min_n", 65) && p.n <= 512)
+        return launch_potrs_cta_strided(p.n, p.nrhs, p.L, p.ldl, p.sl, p.B, p.ldb, p.sb, p.X, p.ldx, p.sx, p.batch,
+                                        stream);
     // "posv.variant": CTA size and the occupancy the register allocation is bounded for (4: as 3,
     // with one column of load look-ahead in the factorisation's tile updates).
     // Measured on GB300 at n = 48 (50,000 instances): 32 threads x 12 CTAs/SM is fastest
@@ -896,7 +851,17 @@ int blastgpu_dposv_mirror_strided(int n, int nrhs, const double* A, int lda, int
     PosvArgs const p{n, nrhs, A, lda, stride_a, L_work, n, (int64_t)n * n, B, ldb, stride_b, X_work, n,
                      (int64_t)n * nrhs, info, batch, 1};
     MirrorOut const o{L, ldl, stride_l, X, ldx, stride_x};
-    posv_mirror_kernel<<<(unsigned)blocks, 32, 0, s>>>(p, o);
+    if (n < kFixMinN || n > 512) {
+        posv_mirror_kernel<true><<<(unsigned)blocks, 32, 0, s>>>(p, o);
+        return check_launch();
+    }
+    if (n <= kPairMaxN)  // the working copy is shared memory
+        return launch_posv_pair(n, nrhs, A, lda, stride_a, L, ldl, stride_l, B, ldb, stride_b, X, ldx, stride_x, info,
+                                batch, s);
+    int const st = launch_potrf_fix(n, A, lda, stride_a, L, ldl, stride_l, L_work, n, (int64_t)n * n, L_work, n,
+                                    (int64_t)n * n, info, batch, s);
+    if (st != BLASTGPU_SUCCESS || nrhs == 0) return st;
+    posv_mirror_kernel<false><<<(unsigned)blocks, 32, 0, s>>>(p, o);
     return check_launch();
 }
 
@@ -924,31 +889,12 @@ int blastgpu_dsyrk_potrf_strided(int n, int k, int trans_a, double alpha, const 
         }
         return BLASTGPU_SUCCESS;
     }
-    // Two implementations with the same bits: syrkLower's warp-per-instance kernel followed by the
-    // thread-per-matrix potrf, or the fused thread-per-matrix kernel, which never stores the sum
-    // but runs the syrk part at thread-per-matrix granularity (1,563 warps for 50,000 instances,
-    // unevenly spread over the 608 sub-partitions). Measured on GB300 at n = 60, k = 30, alpha = 1:
-    // 8.85 ms for the pair vs 9.42 ms fused at 50,000 instances, and the pair is further ahead at
-    // smaller batches, so the pair is the default; "syrk_potrf.fused_min_batch" selects the fused
-    // kernel from that batch size on.
-    // Sizes that the potrf entry point sends to the CTA kernels always take the pair, so that the
-    // result stays equal to syrkLower followed by potrf bit for bit.
-    if (batch < tune_get("syrk_potrf.fused_min_batch", 0x7fffffff) || n >= tune_get("posv.cta_min_n", 65)) {
-        int st = launch_syrk_lower(n, k, trans_a, alpha, A, lda, stride_a, beta, C, ldc, stride_c, D, ldd,
-                                   stride_d, batch, s);
-        if (st != BLASTGPU_SUCCESS) return st;
-        PosvArgs const q{n, 0, D, ldd, stride_d, D, ldd, stride_d, nullptr, 1, 0, nullptr, 1, 0, info, batch, 0};
-        return launch_posv(q, s);
-    }
-    int64_t const blocks = (batch + 31) / 32;
-    if (blocks > 0x7fffffff) return BLASTGPU_ERR_TOO_LARGE;
-    SyrkPotrfArgs const p{n, k, trans_a, alpha, beta, A, lda, stride_a, C, ldc, stride_c, D, ldd, stride_d, info,
-                          batch};
-    if (alpha == 1.0)
-        syrk_potrf_thread_kernel<true><<<(unsigned)blocks, 32, 0, s>>>(p);
-    else
-        syrk_potrf_thread_kernel<false><<<(unsigned)blocks, 32, 0, s>>>(p);
-    return check_launch();
+    // syrkLower's warp-per-instance kernel, then potrf in place.
+    int const st = launch_syrk_lower(n, k, trans_a, alpha, A, lda, stride_a, beta, C, ldc, stride_c, D, ldd, stride_d,
+                                     batch, s);
+    if (st != BLASTGPU_SUCCESS) return st;
+    PosvArgs const q{n, 0, D, ldd, stride_d, D, ldd, stride_d, nullptr, 1, 0, nullptr, 1, 0, info, batch, 0};
+    return launch_posv(q, s);
 }
 
 }  // extern "C"
