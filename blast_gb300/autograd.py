@@ -25,12 +25,24 @@ def _colmajor_copy(t: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def _bwd_call(records: np.ndarray, count: int, max_n: int, recompute: bool, device) -> torch.Tensor:
+def _batch_records(t: torch.Tensor) -> np.ndarray:
+    """Descriptors of the matrices of a column-major (batch, rows, cols) tensor."""
+    out = np.zeros(t.shape[0], dtype=desc.MAT_DTYPE)
+    if len(out):
+        out[:] = np.array(desc.mat_record(t[0]), dtype=desc.MAT_DTYPE)
+        out["data"] = t.data_ptr() + np.arange(len(out)) * (t.stride(0) * t.element_size())
+    return out
+
+
+def _bwd_call(mats, max_n: int, recompute: bool, device):
+    """blastgpu_dposv_bwd_batched on descriptors of A, L, X, Xbar, Bbar and Abar. The descriptors are freed
+    in stream order, after the launch."""
+    records = np.zeros(len(mats[0]), dtype=desc.POSV_BWD_DTYPE)
+    for key, m in zip(desc.POSV_BWD_DTYPE.names, mats):
+        records[key] = m
     d = desc.upload(records, device)
-    info = torch.zeros(count, dtype=torch.int32, device=device)
-    _lib.call("blastgpu_dposv_bwd_batched", d.data_ptr(), count, max_n, int(recompute),
-              info.data_ptr(), torch.cuda.current_stream().cuda_stream)
-    return info, d
+    _lib.call("blastgpu_dposv_bwd_batched", d.data_ptr(), len(records), max_n, int(recompute), 0,
+              torch.cuda.current_stream().cuda_stream)
 
 
 class SPDSolve(torch.autograd.Function):
@@ -61,13 +73,8 @@ class SPDSolve(torch.autograd.Function):
         GA = col_major((batch,), n, n, dev)
         if not ctx.keep:
             L = col_major((batch,), n, n, dev)
-        recs = np.zeros(batch, dtype=desc.POSV_BWD_DTYPE)
-        for b in range(batch):
-            recs[b] = (desc.mat_record(Ac[b]), desc.mat_record(L[b]), desc.mat_record(X[b]),
-                       desc.mat_record(G[b]), desc.mat_record(GB[b]), desc.mat_record(GA[b]))
-        info_b, _keep = _bwd_call(recs, batch, n, not ctx.keep, dev)
-        torch.cuda.current_stream().synchronize()
-        return GA.clone(), GB.clone(), None
+        _bwd_call([_batch_records(t) for t in (Ac, L, X, G, GB, GA)], n, not ctx.keep, dev)
+        return GA, GB, None
 
 
 def spd_solve(A: torch.Tensor, B: torch.Tensor, keep_factor: bool = True) -> torch.Tensor:
@@ -84,12 +91,12 @@ class PackedSPDSolve(torch.autograd.Function):
         from .ragged import Packed, PosvPlan
 
         dev = A_flat.device
-        A = Packed(ns, ns, dev)
+        A = Packed(ns, ns, dev, zero=False)
         A.buf.copy_(A_flat.detach())
-        B = Packed(ns, rs, dev)
+        B = Packed(ns, rs, dev, zero=False)
         B.buf.copy_(B_flat.detach())
-        X = Packed(ns, rs, dev)
-        L = Packed(ns, ns, dev)
+        X = Packed(ns, rs, dev, zero=False)
+        L = Packed(ns, ns, dev, zero=False)
         plan = PosvPlan(A, B, X, L)
         plan.run()
         ctx.packs = (A, L if keep_factor else None, X)
@@ -103,20 +110,15 @@ class PackedSPDSolve(torch.autograd.Function):
         A, L, X = ctx.packs
         ns, rs, keep = ctx.meta
         dev = Xbar_flat.device
-        G = Packed(ns, rs, dev)
+        G = Packed(ns, rs, dev, zero=False)
         G.buf.copy_(Xbar_flat)
-        GB = Packed(ns, rs, dev)
-        GA = Packed(ns, ns, dev)
+        GB = Packed(ns, rs, dev, zero=False)
+        GA = Packed(ns, ns, dev, zero=False)
         if L is None:
-            L = Packed(ns, ns, dev)
-        count = len(ns)
+            L = Packed(ns, ns, dev, zero=False)
         order = np.argsort(-ns, kind="stable")
-        recs = np.zeros(count, dtype=desc.POSV_BWD_DTYPE)
-        for slot, i in enumerate(order):
-            recs[slot] = (A.record(i), L.record(i), X.record(i), G.record(i), GB.record(i), GA.record(i))
-        _bwd_call(recs, count, int(ns.max()), not keep, dev)
-        torch.cuda.current_stream().synchronize()
-        return GA.buf.clone(), GB.buf.clone(), None, None, None
+        _bwd_call([p.records()[order] for p in (A, L, X, G, GB, GA)], int(ns.max()), not keep, dev)
+        return GA.buf, GB.buf, None, None, None
 
 
 def spd_solve_packed(A_flat, B_flat, ns, rs, keep_factor: bool = True) -> torch.Tensor:

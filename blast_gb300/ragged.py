@@ -15,7 +15,7 @@ from . import _lib, desc
 class Packed:
     """Column-major n_i x c_i matrices packed back to back (ld = n_i) in one float64 buffer."""
 
-    def __init__(self, rows, cols, device, dtype=torch.float64):
+    def __init__(self, rows, cols, device, dtype=torch.float64, zero=True):
         self.rows = np.asarray(rows, dtype=np.int64)
         self.cols = np.asarray(cols, dtype=np.int64)
         sizes = self.rows * self.cols
@@ -23,7 +23,7 @@ class Packed:
         if len(sizes):
             self.offsets[1:] = np.cumsum(sizes)[:-1]
         total = int(sizes.sum()) if len(sizes) else 0
-        self.buf = torch.zeros(max(total, 1), dtype=dtype, device=device)
+        self.buf = (torch.zeros if zero else torch.empty)(max(total, 1), dtype=dtype, device=device)
 
     def __len__(self):
         return len(self.rows)
@@ -40,6 +40,16 @@ class Packed:
         r, c = int(self.rows[i]), int(self.cols[i])
         return (self.ptr(i), r, c, max(r, 1), 0, 0, 0)
 
+    def ptrs(self) -> np.ndarray:
+        """The instances' addresses."""
+        return self.buf.data_ptr() + self.offsets * self.buf.element_size()
+
+    def records(self) -> np.ndarray:
+        """record(i) of every instance, as one array."""
+        out = np.zeros(len(self), dtype=desc.MAT_DTYPE)
+        out["data"], out["rows"], out["cols"], out["ld"] = self.ptrs(), self.rows, self.cols, np.maximum(self.rows, 1)
+        return out
+
     def fill_from(self, mats):
         """Copies host matrices (numpy, shapes (rows_i, cols_i)) into the buffer."""
         host = np.zeros(self.buf.numel())
@@ -55,6 +65,15 @@ class Packed:
             r, c, o = int(self.rows[i]), int(self.cols[i]), int(self.offsets[i])
             out.append(host[o:o + r * c].reshape(c, r).T)
         return out
+
+
+def _workspace_offsets(fn, n: np.ndarray, order: np.ndarray):
+    """(byte offset per instance, total bytes) of workspaces of fn(n_i) bytes each, laid out in `order`."""
+    sizes, at = np.unique(n, return_inverse=True)
+    per = np.array([fn(int(k)) for k in sizes], dtype=np.int64)[at] if len(n) else np.zeros(0, dtype=np.int64)
+    off = np.zeros(len(n), dtype=np.int64)
+    off[order] = np.cumsum(per[order]) - per[order]
+    return off, int(per.sum())
 
 
 class PosvPlan:
@@ -79,17 +98,13 @@ class PosvPlan:
         device = A.buf.device
         self.order = np.argsort(-n, kind="stable")  # largest first
         recs = np.zeros(self.count, dtype=desc.POSV_DTYPE)
-        ws_total = 0
-        ws_off = np.zeros(self.count, dtype=np.int64)
+        for key, p in (("A", A), ("L", L), ("B", B), ("X", X)):
+            recs[key] = p.records()[self.order] if p is not None else np.array(desc.EMPTY_MAT, dtype=desc.MAT_DTYPE)
+        self.workspace = None
         if mixed:
-            per = np.array([_lib.lib().blastgpu_dposv_mixed_workspace_bytes(int(k)) for k in n], dtype=np.int64)
-            ws_off[self.order] = np.concatenate([[0], np.cumsum(per[self.order])[:-1]]) if self.count else []
-            ws_total = int(per.sum())
-        self.workspace = torch.empty(max(ws_total, 256), dtype=torch.uint8, device=device) if mixed else None
-        empty = desc.EMPTY_MAT
-        for slot, i in enumerate(self.order):
-            recs[slot] = (A.record(i), L.record(i) if L is not None else empty, B.record(i), X.record(i),
-                          int(ws_off[i]))
+            off, total = _workspace_offsets(_lib.lib().blastgpu_dposv_mixed_workspace_bytes, n, self.order)
+            recs["ws_offset"] = off[self.order]
+            self.workspace = torch.empty(max(total, 256), dtype=torch.uint8, device=device)
         self.d = desc.upload(recs, device)
         self.info = torch.zeros(self.count, dtype=torch.int32, device=device)
         self.iters = torch.zeros(self.count, dtype=torch.int32, device=device)
@@ -179,14 +194,11 @@ class MixedGesvPlan:
         device = A.buf.device
         self.order = np.argsort(-n, kind="stable")
         self.ipiv = Packed(n, np.ones_like(n), device, dtype=torch.int32)
-        per = np.array([_lib.lib().blastgpu_dgesv_mixed_workspace_bytes(int(k)) for k in n], dtype=np.int64)
-        ws_off = np.zeros(self.count, dtype=np.int64)
-        if self.count:
-            ws_off[self.order] = np.concatenate([[0], np.cumsum(per[self.order])[:-1]])
-        self.workspace = torch.empty(max(int(per.sum()), 256), dtype=torch.uint8, device=device)
+        off, total = _workspace_offsets(_lib.lib().blastgpu_dgesv_mixed_workspace_bytes, n, self.order)
+        self.workspace = torch.empty(max(total, 256), dtype=torch.uint8, device=device)
         recs = np.zeros(self.count, dtype=desc.GESV_MIXED_DTYPE)
-        for slot, i in enumerate(self.order):
-            recs[slot] = (A.record(i), self.ipiv.ptr(i), B.record(i), int(ws_off[i]))
+        recs["A"], recs["B"] = A.records()[self.order], B.records()[self.order]
+        recs["ipiv"], recs["ws_offset"] = self.ipiv.ptrs()[self.order], off[self.order]
         self.d = desc.upload(recs, device)
         self.info = torch.zeros(self.count, dtype=torch.int32, device=device)
         self.iters = torch.zeros(self.count, dtype=torch.int32, device=device)
@@ -244,8 +256,7 @@ class GesvPlan:
         self.order = np.argsort(-n, kind="stable")
         self.ipiv = Packed(n, np.ones_like(n), device, dtype=torch.int32)
         recs = np.zeros(self.count, dtype=desc.GETRF_DTYPE)
-        for slot, i in enumerate(self.order):
-            recs[slot] = (A.record(i), self.ipiv.ptr(i), B.record(i))
+        recs["A"], recs["ipiv"], recs["B"] = A.records()[self.order], self.ipiv.ptrs()[self.order], B.records()[self.order]
         self.d = desc.upload(recs, device)
         self.info = torch.zeros(self.count, dtype=torch.int32, device=device)
         self._keep = (A, B)
