@@ -21,7 +21,12 @@ namespace blastgpu {
 namespace {
 
 constexpr int kWarps = 4;    // warps (instances) per CTA
-constexpr int kKChunk = 16;  // K columns staged per pass (static shared memory stays under 48 KB)
+// K columns staged per pass: static shared memory stays under 48 KB, and the loads in flight within the
+// registers of the CTAs below (32 columns took 508 instead of 359 us for 3,000 products of 57 x 39 x 23).
+constexpr int kKChunk = 16;
+// CTAs per SM that a tile's registers are bounded for.
+template <int RM, int RN>
+constexpr int kCtas = RM * RN <= 2 ? 9 : RM * RN <= 4 ? 7 : RM * RN <= 8 ? 6 : 4;
 
 struct StridedGemm {
     int m, n, k;
@@ -108,15 +113,64 @@ __global__ void __launch_bounds__(128) gemm_bwd_c_kernel(const blastgpu_gemm_bwd
     }
 }
 
+// Stages the W x KC panel of an operand whose element (r, q) (r along the tile, q along k) is V(r0 + r,
+// q0 + q), or V(q0 + q, r0 + r) with SWAP, into dst[q][r]; zeros past `rows`. Lanes take consecutive elements
+// of the storage. Elements with q >= kn are left alone.
+template <int W, int KC, bool SWAP>
+__device__ __forceinline__ void stage_panel(double (*dst)[W], MatView const& V, int r0, int q0, int rows, int kn, int lane) {
+    if (V.layout == BLASTGPU_PANEL) {
+        for (int idx = lane; idx < W * KC; idx += 32) {
+            int const r = idx % W, q = idx / W;
+            if (q < kn) dst[q][r] = r0 + r < rows ? (SWAP ? V(q0 + q, r0 + r) : V(r0 + r, q0 + q)) : 0.0;
+        }
+        return;
+    }
+    int64_t const ld = V.ld;
+    if ((V.layout == BLASTGPU_COL_MAJOR) != SWAP) {  // r contiguous
+        constexpr int Q = W >= 32 ? 1 : 32 / W, RS = W >= 32 ? W / 32 : 1;  // columns a pass, passes a column
+        if constexpr (W % 32 == 0 || 32 % W == 0) {
+            int const r = lane % W, q = lane / W;
+            double const* p = V.p + r0 + r + (q0 + q) * ld;
+#pragma unroll
+            for (int s = 0; s < KC / Q; ++s)
+#pragma unroll
+                for (int h = 0; h < RS; ++h)
+                    if (q + s * Q < kn) dst[q + s * Q][r + 32 * h] = r0 + r + 32 * h < rows ? p[s * Q * ld + 32 * h] : 0.0;
+        } else {
+            for (int idx = lane; idx < W * kn; idx += 32) {
+                int const r = idx % W, q = idx / W;
+                dst[q][r] = r0 + r < rows ? V.p[r0 + r + (q0 + q) * ld] : 0.0;
+            }
+        }
+    } else if (kn > 8) {  // q contiguous, 16 lanes to a row
+        int const q = lane % KC, r = lane / KC;
+        double const* p = V.p + q0 + q + (r0 + r) * ld;
+        if (q < kn) {
+#pragma unroll
+            for (int s = 0; s < W / 2; ++s) dst[q][r + 2 * s] = r0 + r + 2 * s < rows ? p[2 * s * ld] : 0.0;
+        }
+    } else {  // 8 lanes
+        int const q = lane % 8, r = lane / 8;
+        double const* p = V.p + q0 + q + (r0 + r) * ld;
+        if (q < kn) {
+#pragma unroll
+            for (int s = 0; s < W / 4; ++s) dst[q][r + 4 * s] = r0 + r + 4 * s < rows ? p[4 * s * ld] : 0.0;
+        }
+    }
+}
+
+// An instance's output tiles are dealt out to `parts` warps (1 when the batch fills the chip by itself).
 template <int RM, int RN, class Batch>
-__global__ void __launch_bounds__(kWarps * 32) gemm_warp_kernel(Batch batch, int64_t count) {
-    constexpr int WM = 4 * RM, WN = 8 * RN;
-    __shared__ double sA[kWarps][kKChunk][WM];
-    __shared__ double sB[kWarps][kKChunk][WN];
+__global__ void __launch_bounds__(kWarps * 32, kCtas<RM, RN>) gemm_warp_kernel(Batch batch, int64_t count, int parts) {
+    constexpr int WM = 4 * RM, WN = 8 * RN, KC = kKChunk;
+    __shared__ __align__(16) double sA[kWarps][KC][WM];
+    __shared__ __align__(16) double sB[kWarps][KC][WN];
 
     int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int64_t const b = (int64_t)blockIdx.x * kWarps + warp;
+    int64_t const w = (int64_t)blockIdx.x * kWarps + warp;
+    int64_t const b = parts == 1 ? w : w / parts;
     if (b >= count) return;
+    int const part = (int)(w - b * parts);
 
     int M, N, K;
     double alpha, beta;
@@ -127,78 +181,131 @@ __global__ void __launch_bounds__(kWarps * 32) gemm_warp_kernel(Batch batch, int
     double (*a_s)[WM] = sA[warp];
     double (*b_s)[WN] = sB[warp];
 
-    for (int ti = 0; ti < M; ti += WM) {
-        for (int tj = 0; tj < N; tj += WN) {
-            double acc[RM][RN];
+    constexpr bool kEarly = RM * RN <= 4;
+    bool const dense = C.layout == BLASTGPU_COL_MAJOR && D.layout == BLASTGPU_COL_MAJOR;
+    int const tm = (M + WM - 1) / WM, tn = (N + WN - 1) / WN;
+    int mi = part % max(tm, 1), nj = part / max(tm, 1);
+    while (nj < tn && tm > 0) {
+        int const ti = mi * WM, tj = nj * WN, i0 = ti + lr * RM, j0 = tj + lc * RN;
+        double ce[RM][RN];  // C, loaded ahead of the products in small tiles
+        if (kEarly && dense) {
 #pragma unroll
-            for (int r = 0; r < RM; ++r)
+            for (int c = 0; c < RN; ++c)
 #pragma unroll
-                for (int c = 0; c < RN; ++c) acc[r][c] = 0.0;
+                for (int r = 0; r < RM; ++r)
+                    ce[r][c] = j0 + c < N && i0 + r < M ? C.p[i0 + r + (int64_t)(j0 + c) * C.ld] : 0.0;
+        }
+        double acc[RM][RN];
+#pragma unroll
+        for (int r = 0; r < RM; ++r)
+#pragma unroll
+            for (int c = 0; c < RN; ++c) acc[r][c] = 0.0;
 
-            for (int kc = 0; kc < K; kc += kKChunk) {
-                int const kn = min(kKChunk, K - kc);
-                __syncwarp();
-                // Stage A(ti:ti+WM, kc:kc+kn): consecutive lanes take consecutive rows.
-                for (int idx = lane; idx < WM * kn; idx += 32) {
-                    int const r = idx % WM, q = idx / WM;
-                    a_s[q][r] = (ti + r < M) ? A(ti + r, kc + q) : 0.0;
-                }
-                // Stage B(kc:kc+kn, tj:tj+WN): consecutive lanes take consecutive k.
-                for (int idx = lane; idx < WN * kn; idx += 32) {
-                    int const q = idx % kn, c = idx / kn;
-                    b_s[q][c] = (tj + c < N) ? B(kc + q, tj + c) : 0.0;
-                }
-                __syncwarp();
-                for (int q = 0; q < kn; ++q) {
-                    double av[RM], bv[RN];
+        for (int kc = 0; kc < K; kc += KC) {
+            int const kn = min(KC, K - kc);
+            __syncwarp();
+            stage_panel<WM, KC, false>(a_s, A, ti, kc, M, kn, lane);
+            stage_panel<WN, KC, true>(b_s, B, tj, kc, N, kn, lane);
+            __syncwarp();
+#pragma unroll 4
+            for (int q = 0; q < kn; ++q) {
+                double av[RM], bv[RN];
 #pragma unroll
-                    for (int r = 0; r < RM; ++r) av[r] = a_s[q][lr * RM + r];
+                for (int r = 0; r < RM; ++r) av[r] = a_s[q][lr * RM + r];
 #pragma unroll
-                    for (int c = 0; c < RN; ++c) bv[c] = b_s[q][lc * RN + c];
+                for (int c = 0; c < RN; ++c) bv[c] = b_s[q][lc * RN + c];
 #pragma unroll
-                    for (int c = 0; c < RN; ++c)
+                for (int c = 0; c < RN; ++c)
 #pragma unroll
-                        for (int r = 0; r < RM; ++r) acc[r][c] = fma(av[r], bv[c], acc[r][c]);
-                }
-            }
-            // Epilogue: acc *= alpha; d = fma(beta, c, acc).
-#pragma unroll
-            for (int c = 0; c < RN; ++c) {
-                int const j = tj + lc * RN + c;
-                if (j < N) {
-#pragma unroll
-                    for (int r = 0; r < RM; ++r) {
-                        int const i = ti + lr * RM + r;
-                        if (i < M) D(i, j) = fma(beta, C(i, j), acc[r][c] * alpha);
-                    }
-                }
+                    for (int r = 0; r < RM; ++r) acc[r][c] = fma(av[r], bv[c], acc[r][c]);
             }
         }
+        // Epilogue: acc *= alpha (exact, and left out, for 1); d = fma(beta, c, acc).
+        if (alpha != 1.0) {
+#pragma unroll
+            for (int c = 0; c < RN; ++c)
+#pragma unroll
+                for (int r = 0; r < RM; ++r) acc[r][c] *= alpha;
+        }
+        if (dense) {
+            double* d = D.p + i0 + (int64_t)j0 * D.ld;
+#pragma unroll
+            for (int c = 0; c < RN; ++c)
+#pragma unroll
+                for (int r = 0; r < RM; ++r)
+                    if (j0 + c < N && i0 + r < M) {
+                        double const cv = kEarly ? ce[r][c] : C.p[i0 + r + (int64_t)(j0 + c) * C.ld];
+                        d[r + (int64_t)c * D.ld] = fma(beta, cv, acc[r][c]);
+                    }
+        } else {
+#pragma unroll
+            for (int c = 0; c < RN; ++c)
+#pragma unroll
+                for (int r = 0; r < RM; ++r)
+                    if (j0 + c < N && i0 + r < M) D(i0 + r, j0 + c) = fma(beta, C(i0 + r, j0 + c), acc[r][c]);
+        }
+        mi += parts;
+        while (mi >= tm) mi -= tm, ++nj;
     }
 }
 
-template <class Batch>
-int launch_gemm(Batch const& batch, int64_t count, int max_m, int max_n, cudaStream_t stream) {
-    if (count == 0) return BLASTGPU_SUCCESS;
-    int64_t const blocks64 = (count + kWarps - 1) / kWarps;
-    if (blocks64 > 0x7fffffff) return BLASTGPU_ERR_TOO_LARGE;
-    dim3 const grid((unsigned)blocks64), block(kWarps * 32);
-    // Warp-tile shape per size bin: by default the smallest tile that covers the instance
-    // without idle lanes where possible (24 x 24 is covered exactly by RM = 6, RN = 3); the
-    // autotuner may override it per bin (0 = 8x8, 1 = 16x16, 2 = 24x24, 3 = 32x32 warp tiles).
-    int const mx = max_m > max_n ? max_m : max_n;
-    int const dflt = (max_m <= 8 && max_n <= 8) ? 0 : (max_m <= 16 && max_n <= 16) ? 1
-                   : (max_m <= 24 && max_n <= 24) ? 2 : 3;
-    // gemm tiles change every 8 rows/columns, so its bins are multiples of 8 ("gemm.shape.m24").
-    char key[32];
-    snprintf(key, sizeof(key), "gemm.shape.m%d", ((mx + 7) / 8) * 8);
-    switch (tune_get(key, dflt)) {
-        case 0: gemm_warp_kernel<2, 1><<<grid, block, 0, stream>>>(batch, count); break;
-        case 1: gemm_warp_kernel<4, 2><<<grid, block, 0, stream>>>(batch, count); break;
-        case 2: gemm_warp_kernel<6, 3><<<grid, block, 0, stream>>>(batch, count); break;
-        default: gemm_warp_kernel<8, 4><<<grid, block, 0, stream>>>(batch, count); break;
-    }
+template <int RM, int RN, class Batch>
+int launch_shape(Batch const& batch, int64_t count, int parts, cudaStream_t stream) {
+    int64_t const blocks = (count * parts + kWarps - 1) / kWarps;
+    if (blocks > 0x7fffffff) return BLASTGPU_ERR_TOO_LARGE;
+    gemm_warp_kernel<RM, RN><<<(unsigned)blocks, kWarps * 32, 0, stream>>>(batch, count, parts);
     return check_launch();
+}
+
+// The warp tile (0 = 8 x 8, 1 = 16 x 16, 2 = 24 x 24, 3 = 16 x 8) and whether an instance's tiles go to one
+// warp or to a warp each, by the multiply-adds that the busiest scheduler gets. A tile without padding runs
+// at 0.83 (8 x 8) to 0.90 (24 x 24) of the binary64 rate, since a larger tile has fewer loads per
+// multiply-add, and a warp costs a dozen multiply-adds to start. Padding, and warps that do not divide
+// evenly among the schedulers, cost in full. Measured: 24 x 24 x 24 x 10,000 in one tile 255 us, in 8 x 8 tiles
+// 278 us; 57 x 39 x 23 x 3,000 in 8 x 8 tiles 354 us, in 24 x 24 453 us; 75 x 66 x 64 x 4,586 in 16 x 8 tiles 2.86 ms,
+// in 8 x 8 3.24 ms; one 128 x 128 x 128 a warp a tile 25 us, one warp 4.6 ms. 32 x 32 tiles were never ahead.
+struct Choice {
+    int shape, parts;
+};
+Choice choose(int64_t count, int m, int n, int k, int only) {
+    static constexpr struct { int wm, wn; double rate; } kShapes[] = {
+        {8, 8, 0.83}, {16, 16, 0.87}, {24, 24, 0.90}, {16, 8, 0.845}};
+    int64_t const schedulers = 4 * (int64_t)sm_count();
+    Choice best{0, 1};
+    double cost = 1e300;
+    for (int s = 0; s < 4; ++s) {
+        if (only >= 0 && s != only) continue;
+        int64_t const tiles = (int64_t)((m + kShapes[s].wm - 1) / kShapes[s].wm) * ((n + kShapes[s].wn - 1) / kShapes[s].wn);
+        double const tile = kShapes[s].wm * kShapes[s].wn / 32.0 * (k + 2) / kShapes[s].rate;
+        for (int split = 0; split < 2; ++split) {
+            int64_t const parts = split ? tiles : 1;
+            int64_t const rounds = (count * parts + schedulers - 1) / schedulers;
+            double const c = rounds * (tile * (tiles / parts) + 12);
+            if (c < cost && parts <= 0x7fffffff) cost = c, best = {s, (int)parts};
+        }
+    }
+    return best;
+}
+
+template <class Batch>
+int launch_gemm(Batch const& batch, int64_t count, int max_m, int max_n, int max_k, cudaStream_t stream) {
+    if (count == 0 || max_m == 0 || max_n == 0) return BLASTGPU_SUCCESS;
+    if (count > 0x7fffffffll * kWarps) return BLASTGPU_ERR_TOO_LARGE;
+    // The autotuner's choice for a square bin, "gemm.shape.m24": sizes that round up to the same multiple of 8.
+    int only = -1;
+    if ((max_m + 7) / 8 == (max_n + 7) / 8) {
+        char key[32];
+        snprintf(key, sizeof(key), "gemm.shape.m%d", ((max_m + 7) / 8) * 8);
+        only = tune_get(key, -1);
+        if (only > 3) only = -1;
+    }
+    Choice const c = choose(count, max_m, max_n, max_k, only);
+    switch (c.shape) {
+        case 0: return launch_shape<2, 1>(batch, count, c.parts, stream);
+        case 1: return launch_shape<4, 2>(batch, count, c.parts, stream);
+        case 2: return launch_shape<6, 3>(batch, count, c.parts, stream);
+        default: return launch_shape<4, 1>(batch, count, c.parts, stream);
+    }
 }
 
 }  // namespace
@@ -236,7 +343,7 @@ int blastgpu_dgemm_strided(int trans_a, int trans_b, int m, int n, int k, double
     g.C = MatView{const_cast<double*>(C), ldc, BLASTGPU_COL_MAJOR, 1};
     g.D = MatView{D, ldd, BLASTGPU_COL_MAJOR, 1};
     g.sa = stride_a; g.sb = stride_b; g.sc = stride_c; g.sd = stride_d;
-    return launch_gemm(g, batch, m, n, as_cuda(stream));
+    return launch_gemm(g, batch, m, n, k, as_cuda(stream));
 }
 
 int blastgpu_dgemm_bwd_batched(const blastgpu_gemm_bwd_desc* desc, int64_t batch, int max_dim, int32_t* status,
@@ -251,9 +358,9 @@ int blastgpu_dgemm_bwd_batched(const blastgpu_gemm_bwd_desc* desc, int64_t batch
     gemm_bwd_c_kernel<<<(unsigned)blocks, 128, 0, s>>>(desc, batch, status);
     int st = check_launch();
     if (st != BLASTGPU_SUCCESS) return st;
-    st = launch_gemm(GemmBwdBatch{desc, 0}, batch, max_dim, max_dim, s);
+    st = launch_gemm(GemmBwdBatch{desc, 0}, batch, max_dim, max_dim, max_dim, s);
     if (st != BLASTGPU_SUCCESS) return st;
-    return launch_gemm(GemmBwdBatch{desc, 1}, batch, max_dim, max_dim, s);
+    return launch_gemm(GemmBwdBatch{desc, 1}, batch, max_dim, max_dim, max_dim, s);
 }
 
 int blastgpu_dgemm_batched(const blastgpu_gemm_desc* desc, int64_t batch, int max_m, int max_n,
@@ -265,7 +372,7 @@ int blastgpu_dgemm_batched(const blastgpu_gemm_desc* desc, int64_t batch, int ma
     if (max_n < 0) return -4;
     if (max_k < 0) return -5;
     DescGemm g{desc};
-    return launch_gemm(g, batch, max_m, max_n, as_cuda(stream));
+    return launch_gemm(g, batch, max_m, max_n, max_k, as_cuda(stream));
 }
 
 }  // extern "C"

@@ -5,8 +5,8 @@ Tunable choices (read by the library through blastgpu_tune_set / tune_get_bin):
 * ``posv.variant.n<bin>`` — thread-per-matrix Cholesky solve: CTA size and the register budget
   the kernel is compiled for (0: 64 threads, 213 registers; 1: 64 x 168; 2: 128 x 168;
   3: 32 x 168; 4: 32 x 168 with one column of load look-ahead in the tile updates).
-* ``gemm.shape.m<8k>`` — warp tile of the batched gemm (0: 8x8, 1: 16x16, 2: 24x24, 3: 32x32),
-  per largest dimension rounded up to a multiple of 8.
+* ``gemm.shape.m<8k>`` — warp tile of the batched gemm (0: 8x8, 1: 16x16, 2: 24x24, 3: 16x8) where both
+  dimensions of D round up to this multiple of 8; without it the library weighs the tiles by their padding.
 * ``getrf.cta.n<bin>`` — ragged LU: one warp (0) or one 256-thread CTA (1) per matrix, per size bin
   of the launch's largest n (same bits either way).
 * ``getrf.lazy.n<bin>`` — the CTA kernel's schedule: right-looking (0) or left-looking with the left

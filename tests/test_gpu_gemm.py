@@ -103,3 +103,23 @@ def test_gemm_in_place_and_errors(gpu, oracle_lib):
     assert np.array_equal(dC.cpu().numpy(), ref)
     with pytest.raises(ValueError, match="Matrix sizes do not match"):
         gpu.gemm(to_dev(A[:, :, :5]), to_dev(B), dC, dC)
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(1, 1, 1, 1), (8, 8, 16, 3), (9, 17, 33, 2), (16, 8, 16, 700), (24, 24, 24, 2500),
+                                         (25, 24, 17, 40), (49, 50, 5, 9), (130, 3, 40, 1), (48, 48, 9, 30),
+                                         (17, 33, 8, 1300), (5, 130, 24, 2)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, True), (True, False)])
+def test_gemm_tiles_and_splits(gpu, oracle_lib, m, n, k, batch, ta, tb):
+    """Every warp tile, whole instances per warp and tiles dealt out to warps, each storage order: the
+    oracle's bits, whatever the library chooses."""
+    import torch
+
+    rng = np.random.default_rng(m * 1000 + n)
+    A, B, C = (rng.uniform(-1, 1, (batch, *s)) for s in ((m, k), (k, n), (m, n)))
+    ref = oracle_lib.gemm_batch(1.0 if ta else 0.3, A, B, -0.5, C)
+    dA = torch.from_numpy(A).cuda() if ta else to_dev(A)
+    dB = torch.from_numpy(B).cuda() if tb else to_dev(B)
+    dC = to_dev(C)
+    gpu.gemm(1.0 if ta else 0.3, dA, dB, -0.5, dC, dC)
+    torch.cuda.synchronize()
+    assert np.array_equal(dC.cpu().numpy(), ref)
