@@ -78,6 +78,81 @@ __global__ void __launch_bounds__(128) trsm_kernel(int uplo, int trans_a, int un
     }
 }
 
+// trsm with the solution in shared memory: one thread per (instance, right-hand-side column), a warp per
+// CTA. Each column is one chain of fused multiply-adds in BLAST's order (for the upper triangle the newest
+// entry comes first, so nothing can be summed ahead), and a warp holds its scheduler's binary64 pipe for
+// the whole of a step; what the chain must not wait for is memory. B arrives and X leaves in whole columns,
+// x is read without bank conflicts (stride 33), and the triangle's entries are loaded 8 terms ahead, the
+// next row's first ones included.
+constexpr int kTrsmAhead = 8;
+
+__global__ void __launch_bounds__(32) trsm_shared_kernel(int uplo, int trans_a, int unit, int m, int n, Strided A, Strided B,
+                                                         Strided X, int64_t columns) {
+    extern __shared__ double x[];  // [m][33]
+    int const lane = threadIdx.x;
+    int64_t const t0 = (int64_t)blockIdx.x * 32, t = t0 + lane;
+    int const cols = (int)min((int64_t)32, columns - t0);
+    {
+        int64_t b = t0 / n;
+        int j = (int)(t0 - b * n);
+#pragma unroll 4
+        for (int c = 0; c < cols; ++c) {
+            for (int i = lane; i < m; i += 32) x[i * 33 + c] = B.at(b, i, j);
+            if (++j == n) j = 0, ++b;
+        }
+    }
+    __syncwarp();
+    if (lane < cols) {
+        double const* a = A.p + (t / n) * A.stride;
+        int64_t const si = trans_a ? A.ld : 1, sq = trans_a ? 1 : A.ld;  // a(i, q) = a[i * si + q * sq]
+        bool const lower = uplo == BLASTGPU_LOWER;
+        double cur[kTrsmAhead], nxt[kTrsmAhead];
+#pragma unroll
+        for (int u = 0; u < kTrsmAhead; ++u) cur[u] = 0.0;
+        for (int s = 0; s < m; ++s) {  // s terms before row i's division
+            int const i = lower ? s : m - 1 - s, q0 = lower ? 0 : i + 1;
+            double acc = x[i * 33 + lane];
+            double const d = unit ? 1.0 : a[i * si + i * sq];
+            int const chunks = max(1, (s + kTrsmAhead - 1) / kTrsmAhead);
+            for (int ch = 0; ch < chunks; ++ch) {
+                // the chunk after this one: of this row, or the first of the next
+                bool const same = ch + 1 < chunks;
+                int const ni = same ? i : lower ? i + 1 : i - 1, nq = same ? q0 + (ch + 1) * kTrsmAhead : lower ? 0 : ni + 1;
+                int const left = same ? s - (ch + 1) * kTrsmAhead : s + 1 < m ? s + 1 : 0;
+#pragma unroll
+                for (int u = 0; u < kTrsmAhead; ++u) nxt[u] = u < left ? a[ni * si + (nq + u) * sq] : 0.0;
+                int const q = q0 + ch * kTrsmAhead, have = s - ch * kTrsmAhead;
+#pragma unroll
+                for (int u = 0; u < kTrsmAhead; ++u)
+                    if (u < have) acc = fma(-cur[u], x[(q + u) * 33 + lane], acc);
+#pragma unroll
+                for (int u = 0; u < kTrsmAhead; ++u) cur[u] = nxt[u];
+            }
+            x[i * 33 + lane] = unit ? acc : acc / d;
+        }
+    }
+    __syncwarp();
+    int64_t b = t0 / n;
+    int j = (int)(t0 - b * n);
+#pragma unroll 4
+    for (int c = 0; c < cols; ++c) {
+        for (int i = lane; i < m; i += 32) X.at(b, i, j) = x[i * 33 + c];
+        if (++j == n) j = 0, ++b;
+    }
+}
+
+// Where that pays. Measured on GB300 (global memory, then shared, us): lower m = 50, n = 6, 5,933 instances: 236, 174;
+// m = 64, n = 16, 2,000: 335, 187 (upper 319, 206); m = 128, n = 64, 300: 703, 460; one upper m = 98, n = 3: 317, 300. Small
+// triangles leave too little to hide the copies behind (m = 22, n = 40, 2,467: 56, 114; upper m = 56, n = 2, 17: 135,
+// 140), and so does a batch whose warps do not fit the SMs' shared memory at once, which reaches the
+// pipe's rate without (m = 102, n = 30, 3,794: 1,169, 1,584).
+bool trsm_shared_wanted(int uplo, int m, int64_t columns) {
+    constexpr int kMaxM = 160;  // 42 KB
+    if (m < (uplo == BLASTGPU_LOWER ? 48 : 64) || m > kMaxM) return false;
+    int64_t const resident = (int64_t)(227 * 1024) / (m * 33 * 8 + 1024);
+    return (columns + 31) / 32 <= resident * sm_count();
+}
+
 template <bool ALPHA1>
 __global__ void __launch_bounds__(128) trmm_kernel(int side, int uplo, int unit, int m, int n, double alpha,
                                                    Strided A, Strided B, Strided C, int64_t batch) {
@@ -187,6 +262,11 @@ int blastgpu_dtrsm_strided(int uplo, int trans_a, int unit, int m, int n, const 
     Strided a{const_cast<double*>(A), lda, stride_a, BLASTGPU_COL_MAJOR};
     Strided bb{const_cast<double*>(B), ldb, stride_b, BLASTGPU_COL_MAJOR};
     Strided x{X, ldx, stride_x, BLASTGPU_COL_MAJOR};
+    if (trsm_shared_wanted(uplo, m, threads)) {
+        trsm_shared_kernel<<<(unsigned)((threads + 31) / 32), 32, (size_t)m * 33 * sizeof(double), as_cuda(stream)>>>(
+            uplo, trans_a, unit, m, n, a, bb, x, threads);
+        return check_launch();
+    }
     trsm_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, as_cuda(stream)>>>(uplo, trans_a, unit, m, n, a, bb, x, batch);
     return check_launch();
 }

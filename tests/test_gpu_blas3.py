@@ -169,3 +169,26 @@ def test_trsm_right_side(gpu, oracle_lib, uplo, unit, trans):
                 if unit:
                     np.fill_diagonal(T, 1.0)
                 assert approx_equal(X[b] @ T, B[b], 1e-10, 1e-10)
+
+
+@pytest.mark.parametrize("m,n,batch", [(47, 3, 2), (48, 5, 3), (63, 32, 1), (64, 1, 40), (65, 33, 2), (160, 2, 3), (161, 2, 2),
+                                       (72, 40, 1300)])
+@pytest.mark.parametrize("uplo,unit,trans", [(0, 0, 0), (1, 0, 1), (0, 1, 1), (1, 1, 0)])
+def test_trsm_shared_and_global(gpu, oracle_lib, m, n, batch, uplo, unit, trans):
+    """Both sides of the sizes and batches that keep the solution in shared memory: the oracle's bits, with
+    X its own array and in place of B, and padded leading dimensions."""
+    import torch
+
+    rng = np.random.default_rng(m * 100 + n)
+    A = rng.random((batch, m, m)) / m + np.eye(m)
+    B = rng.random((batch, m, n))
+    dA = torch.from_numpy(A).cuda() if trans else to_dev(A, ld=m + 1)
+    dB, dX = to_dev(B, ld=m + 2), gpu.col_major((batch,), m, n, "cuda")
+    gpu.trsm(uplo, bool(unit), dA, dB, dX)
+    gpu.trsm(uplo, bool(unit), dA, dB, dB)
+    torch.cuda.synchronize()
+    assert torch.equal(dX, dB)
+    for b in {0, batch // 2, batch - 1}:
+        Xr = F(np.zeros((m, n)))
+        oracle_lib.trsm(uplo, unit, F(A[b]), F(B[b]), Xr)
+        assert np.array_equal(dX[b].cpu().numpy(), Xr), b
