@@ -104,6 +104,12 @@ FIX64_FN int64_t join(Limbs v) {
     return q;
 }
 
+// Digits for the tensor cores: 4 q = sum of d_i 2^(8 (7 - i)), d_i in [-128, 127], kept as the bytes d_i + 128 of
+// one 64-bit word (two bits more than q, so that the digits past the ones that are multiplied weigh less).
+constexpr uint64_t kDigitBias = 0x8080808080808080ull;
+FIX64_FN int64_t to_digits(int64_t q) { return (int64_t)(((uint64_t)q << 2) + kDigitBias); }
+FIX64_FN int64_t from_digits(int64_t u) { return (int64_t)((uint64_t)u - kDigitBias) >> 2; }
+
 // A cross sum starts here, so that total() rounds to nearest.
 constexpr int64_t kCrossStart = int64_t(1) << 29;
 

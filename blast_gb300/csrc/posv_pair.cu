@@ -152,16 +152,23 @@ __device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int col
     }
     bool const no_pivot = bad[l16] != 0;
     bool off = false;
+    // The next pivot's reciprocal square root is taken as soon as its column is up to date, beside the
+    // products of the columns after it.
+    int64_t t = 0;
+    Rsqrt y;
+    auto pivot = [&](int c) {
+        t = acc[c] - fix64::total(0, -cr[c]);
+        int64_t s = __shfl_sync(0xffffffffu, off || no_pivot ? (int64_t)-1 : t, c, kB);
+        if (s < fix64::kPivotMin) {
+            fail = min(fail, first + c);
+            s = int64_t(1) << 60;
+        }
+        y = fix64::pivot_rsqrt(s);
+    };
+    pivot(0);
 #pragma unroll
     for (int j = 0; j < kB; ++j) {
         if (j < cols) {
-            int64_t const t = acc[j] - fix64::total(0, -cr[j]);
-            int64_t s = __shfl_sync(0xffffffffu, off || no_pivot ? (int64_t)-1 : t, j, kB);
-            if (s < fix64::kPivotMin) {
-                fail = min(fail, first + j);
-                s = int64_t(1) << 60;
-            }
-            Rsqrt const y = fix64::pivot_rsqrt(s);
             int64_t q;
             bool const ok = fix64::scale_entry<fix64::kEntryBits>(t, y, q);
             off |= !ok && l16 > j;
@@ -175,6 +182,7 @@ __device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int col
                 fix64::mad(acc[c], nh, h);
                 fix64::mad(cr[c], nh, l);
                 fix64::mad(cr[c], nl, h);
+                if (c == j + 1) pivot(c);
             }
         }
     }

@@ -4,20 +4,27 @@
 // of all earlier columns (the ger(-1, ...) loop), is factored on the diagonal and solved below it.
 //
 // What bounds it: in binary64 the multiply-adds, 2 lanes a clock and SM whatever the mapping (33.6 ms for
-// 2,048 matrices with n uniform in 64 .. 512, factored and solved with one right-hand side). In fixed
-// point the integer multiplications and additions, six instructions a product on two pipes (9.3 ms for
-// the same batch), with the matrix's rows scaled; binary64 is left with one conversion per factor entry.
+// 2,048 matrices with n uniform in 64 .. 512, factored and solved with one right-hand side). In fixed point,
+// with the matrix's rows scaled, the products of earlier columns run on the integer pipe (n <= 128) or on the
+// tensor cores (above), which took the same batch to 9.3 ms and, for its n > 128, to 7.6 ms; binary64 is left
+// with one conversion per factor entry. At n = 512 with three CTAs an SM, three quarters of a CTA's time are
+// the products (tensor pipe 63% busy meanwhile, the rest taking entries apart into digits and waiting for
+// the staged columns), 8% the diagonal blocks, 8% the rows below them, 7% the conversion. At n = 128
+// the products are half, the diagonal blocks' chains a quarter.
 //
 // Mapping: one CTA of T threads per matrix, panels of 16 columns, the rows of a panel in chunks of T.
-//  * Update: each thread holds a 4 x 4 tile of the T x 16 chunk (rows T/4 apart, adjacent columns;
-//    64 registers of sums), the earlier columns come through shared memory 16 at a time, double
-//    buffered with cp.async. A step costs 48 multiply-adds against 4 row loads and 2 (16-byte)
-//    column loads, all free of bank conflicts.
+//  * Products, T = 32 and 64: each thread holds a 4 x 4 tile of the T x 16 chunk (rows T/4 apart, adjacent
+//    columns; 64 registers of sums), the earlier columns come through shared memory 16 at a time, double
+//    buffered with cp.async. A step costs 48 multiply-adds against 4 row loads and 2 (16-byte) column
+//    loads, all free of bank conflicts.
+//  * Products, T = 128: digits of 8 bits on the tensor cores (update_chunk_mma), 32 columns at a time. With
+//    T = 64 this lost to the integer products (n = 128 x 4,000: 2.06 against 1.72 ms): six CTAs an SM for
+//    eight.
 //  * The first chunk's first 32 rows: one warp, a row per lane, the 16 columns right-looking in
 //    registers, the pivot row's limbs by shuffles. The reciprocal square root is integer as well.
 //  * Other rows: a row per thread against the diagonal block, left-looking in registers.
-//  * The factor stays in fixed point in the workspace (L itself, unless the caller says otherwise),
-//    where the later panels read it, and becomes binary64 in one last pass.
+//  * The factor stays in fixed point in the workspace (L itself, unless the caller says otherwise), as
+//    limbs or as digits, where the later panels read it, and becomes binary64 in one last pass.
 //
 // Panels of 16 keep the work inside a panel, which runs at a lower rate, at 8 n^2 of the n^3 / 6
 // products, and let all T threads own a row of it.
@@ -35,11 +42,15 @@ constexpr int kNB = 16;
 template <int T>
 struct Shape {
     static constexpr int NMAX = T == 32 ? 64 : T == 64 ? 128 : 512;  // largest n that runs with T threads
-    static constexpr int RT = T / 4;    // distance of a thread's rows
-    static constexpr int RS = T + kNB;  // staged column: the chunk's rows, then the diagonal block's
-    static constexpr int CS = T + 2;    // column stride of the chunk: 4 columns x 8 rows hit all banks
+    static constexpr bool kTensor = T == 128;  // products on the tensor cores
+    static constexpr int kWarps = T / 32;
+    static constexpr int RT = T / 4;  // distance of a thread's rows in integer products
+    // staged column: the chunk's rows, then the diagonal block's (reads of 8 rows by 2 columns hit all banks)
+    static constexpr int RS = T + kNB + (kTensor ? 4 : 0);
+    static constexpr int CS = T + 2;        // column stride of the chunk's remainders
     static constexpr int kStage = 0;
-    static constexpr int kChunk = kStage + 2 * kNB * RS * 8;
+    static constexpr int kDigits = kStage + 2 * kNB * RS * 8;
+    static constexpr int kChunk = kDigits + (kTensor ? 2 * 8 * kNB * kNB * 2 : 0);
     static constexpr int kDiag = kChunk + kNB * CS * 8;
     static constexpr int kRsqrt = kDiag + kNB * kNB * 8;
     static constexpr int kScale = kRsqrt + kNB * 16;
@@ -53,7 +64,7 @@ __device__ __forceinline__ void cta_sync() {
     else __syncthreads();
 }
 
-__device__ __forceinline__ void cp_async8(Limbs* dst, const Limbs* src) {
+__device__ __forceinline__ void cp_async8(int64_t* dst, const int64_t* src) {
     unsigned const d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
@@ -61,11 +72,11 @@ __device__ __forceinline__ void cp_async8(Limbs* dst, const Limbs* src) {
 // Columns 16 s .. 16 s + 15 of the workspace, rows k0 + r0 .. of the chunk; below the first chunk
 // also the diagonal block's rows.
 template <int T>
-__device__ __forceinline__ void stage_columns(Limbs* stage, const Limbs* W, int64_t ldw, int k0, int r0, int mr, int nb,
+__device__ __forceinline__ void stage_columns(int64_t* stage, const int64_t* W, int64_t ldw, int k0, int r0, int mr, int nb,
                                               int s) {
     using S = Shape<T>;
-    Limbs* dst = stage + (s & 1) * kNB * S::RS;
-    Limbs const* src = W + k0 + (int64_t)(kNB * s) * ldw;
+    int64_t* dst = stage + (s & 1) * kNB * S::RS;
+    int64_t const* src = W + k0 + (int64_t)(kNB * s) * ldw;
     int const tid = threadIdx.x;
     if (tid < mr) {
 #pragma unroll
@@ -80,12 +91,35 @@ __device__ __forceinline__ void stage_columns(Limbs* stage, const Limbs* W, int6
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
+// Digit i (0 the highest) of two entries as a pair of binary16 numbers: the byte becomes the low bits of
+// 1024 + byte, and 1152 is taken off again.
+template <int I>
+__device__ __forceinline__ uint32_t digit_pair(int64_t u0, int64_t u1) {
+    uint32_t const a = I < 4 ? (uint32_t)(u0 >> 32) : (uint32_t)u0, b = I < 4 ? (uint32_t)(u1 >> 32) : (uint32_t)u1;
+    constexpr int kByte = 3 - (I & 3);
+    uint32_t const bytes = __byte_perm(a, b, kByte | kByte << 4 | (4 + kByte) << 8 | (4 + kByte) << 12);
+    uint32_t const biased = (bytes & 0x00ff00ffu) | 0x64006400u;
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(biased), "r"(0x64806480u));
+    return d;
+}
+__device__ __forceinline__ void digit_pairs(uint32_t (&d)[8], int64_t u0, int64_t u1) {
+    d[0] = digit_pair<0>(u0, u1), d[1] = digit_pair<1>(u0, u1), d[2] = digit_pair<2>(u0, u1), d[3] = digit_pair<3>(u0, u1);
+    d[4] = digit_pair<4>(u0, u1), d[5] = digit_pair<5>(u0, u1), d[6] = digit_pair<6>(u0, u1), d[7] = digit_pair<7>(u0, u1);
+}
+
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t const (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
 // The chunk's remainders A - L L^T over the columns before k0, into C (units of 2^-62). RA: rows per
 // thread that the chunk needs. Rows past mr and columns past nb hold whatever shared memory held; they
 // are not used.
 template <int T, int RA>
-__device__ __forceinline__ void update_chunk(int k0, int r0, int mr, int nb, const double* A, int64_t lda,
-                                             const Limbs* W, int64_t ldw, Limbs* stage, int64_t* C, const int* scale,
+__device__ __forceinline__ void update_chunk_int(int k0, int r0, int mr, int nb, const double* A, int64_t lda,
+                                             const int64_t* W, int64_t ldw, int64_t* stage, int64_t* C, const int* scale,
                                              unsigned char* bad) {
     using S = Shape<T>;
     int const lane = threadIdx.x & 31, ct = 4 * (lane >> 3), rt = 8 * (threadIdx.x >> 5) + (lane & 7);
@@ -115,8 +149,8 @@ __device__ __forceinline__ void update_chunk(int k0, int r0, int mr, int nb, con
         }
         if (!ok && r < mr) bad[k0 + r0 + r] = fix64::kNoPivot | fix64::kOutOfRange;
     }
-    Limbs const* colbase = stage + (r0 == 0 ? ct : T + ct);
-    Limbs const* rowbase = stage + rt;
+    int64_t const* colbase = stage + (r0 == 0 ? ct : T + ct);
+    int64_t const* rowbase = stage + rt;
     for (int s = 0; s < slabs; ++s) {
         if (s + 1 < slabs) {
             stage_columns<T>(stage, W, ldw, k0, r0, mr, nb, s + 1);
@@ -133,7 +167,7 @@ __device__ __forceinline__ void update_chunk(int k0, int r0, int mr, int nb, con
             int const bl[4] = {b01.x, b01.z, b23.x, b23.z}, bh[4] = {b01.y, b01.w, b23.y, b23.w};
 #pragma unroll
             for (int i = 0; i < RA; ++i) {
-                Limbs const v = rowbase[base + q * S::RS + S::RT * i];
+                Limbs const v = fix64::unpack(rowbase[base + q * S::RS + S::RT * i]);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     fix64::mad(hh[i][j], v.h, bh[j]);
@@ -160,11 +194,130 @@ __device__ __forceinline__ void update_chunk(int k0, int r0, int mr, int nb, con
     }
 }
 
+// The same on the tensor cores. An entry is 8 digits of 8 bits; the 36 products of digits i + j <= 7 go into 8
+// binary32 accumulators by i + j. All are sums of integers: over 32 columns, 6 products of at most 2^14 and 2
+// of at most 2^13 (an entry's highest digit has 6 bits) a column stay below 2^22, so they are exact, and an
+// accumulator that starts at 1.5 x 2^23 holds its sum in its low mantissa bits. The digits i + j > 7 left out
+// weigh 2^-60 sqrt(columns) in all.
+// Warp w has the row tiles (16 rows) w and w + T/32; lane (g, q) = (lane / 4, lane % 4) of a tile has rows g, g + 8
+// and columns 2 q, 2 q + 1 of each 8 columns. The 16 rows of the diagonal block are taken apart into digits
+// once per 32 columns, by all threads, in fragment order; a row tile's by the warp that has it.
+template <int T>
+__device__ __forceinline__ void update_chunk_mma(int k0, int r0, int mr, int nb, const double* A, int64_t lda,
+                                                 const int64_t* W, int64_t ldw, int64_t* stage, uint4* digits, int64_t* C,
+                                                 const int* scale, unsigned char* bad) {
+    using S = Shape<T>;
+    int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q2 = 2 * (lane & 3);
+    {  // A's entries start towards L2: a column's 128-byte line per thread
+        int const c = tid % kNB, r = 16 * (tid / kNB);
+        if (c < nb && r < mr) asm volatile("prefetch.global.L2 [%0];" ::"l"(A + k0 + r0 + r + (int64_t)(k0 + c) * lda));
+    }
+    int64_t sum[2][2][4];
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[t][n][e] = 0;
+    int const slabs = k0 / kNB;
+    for (int s = 0; s < slabs; s += 2) {
+        int const ns = min(2, slabs - s);
+        for (int u = 0; u < ns; ++u) stage_columns<T>(stage, W, ldw, k0, r0, mr, nb, s + u);
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        cta_sync<T>();
+        for (int e = tid; e < 64 * ns; e += T) {  // slab u, column n of the product, k = 2 q, 2 q + 1, 2 q + 8, 2 q + 9
+            int const u = e >> 6, n = (e >> 2) & 15, q = e & 3;
+            int64_t const* src = stage + (u * kNB + 2 * q) * S::RS + (r0 == 0 ? 0 : T) + n;
+            uint32_t d0[8], d1[8];
+            digit_pairs(d0, src[0], src[S::RS]);
+            digit_pairs(d1, src[8 * S::RS], src[9 * S::RS]);
+            uint4* dst = digits + (u * 2 + (n >> 3)) * 4 * 32 + (n & 7) * 4 + q;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dst[i * 32] = make_uint4(d0[2 * i], d1[2 * i], d0[2 * i + 1], d1[2 * i + 1]);
+        }
+        cta_sync<T>();
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            int const first = 16 * (warp + S::kWarps * t);
+            if (first < mr) {  // warp-uniform
+                float acc[2][8][4];
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[n][i][e] = 12582912.0f;
+#pragma unroll 1
+                for (int u = 0; u < ns; ++u) {
+                    uint32_t a[8][4];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {  // fragment register h: rows g + 8 (h & 1), k = 2 q + 8 (h >> 1)
+                        int64_t const* src = stage + (u * kNB + q2 + 8 * (h >> 1)) * S::RS + first + g + 8 * (h & 1);
+                        uint32_t d[8];
+                        digit_pairs(d, src[0], src[S::RS]);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) a[i][h] = d[i];
+                    }
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) {
+                        uint4 const* dig = digits + (u * 2 + n) * 4 * 32 + lane;
+#pragma unroll
+                        for (int jj = 0; jj < 4; ++jj) {
+                            uint4 const v = dig[jj * 32];
+#pragma unroll
+                            for (int i = 0; i + 2 * jj < 8; ++i) mma_f16(acc[n][i + 2 * jj], a[i], v.x, v.y);
+#pragma unroll
+                            for (int i = 0; i + 2 * jj + 1 < 8; ++i) mma_f16(acc[n][i + 2 * jj + 1], a[i], v.z, v.w);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        constexpr uint32_t kStart = 0x4b400000u;  // the bits of 1.5 x 2^23
+                        int32_t v[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            v[i] = (int32_t)(__float_as_uint(acc[n][2 * i][e]) * 256u +
+                                             (__float_as_uint(acc[n][2 * i + 1][e]) - kStart * 257u));
+                        int64_t hi = v[1], lo = v[3] + 128;  // units of 2^-38 and 2^-70
+                        fix64::mad(hi, v[0], 65536);
+                        fix64::mad(lo, v[2], 65536);
+                        sum[t][n][e] += (hi << 24) + (lo >> 8);
+                    }
+            }
+        }
+        cta_sync<T>();  // the staged columns are written again
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            int const r = 16 * (warp + S::kWarps * t) + g + 8 * h;
+            if (r < mr) {
+                int const er = scale[k0 + r0 + r];
+                bool ok = true;
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        int const c = 8 * n + q2 + e;
+                        int64_t v = 0;
+                        if (c < nb && r0 + r >= c)
+                            ok &= fix64::from_double(A[(k0 + r0 + r) + (int64_t)(k0 + c) * lda], er + scale[k0 + c], v);
+                        C[c * S::CS + r] = v - sum[t][n][2 * h + e];
+                    }
+                if (!ok) bad[k0 + r0 + r] = fix64::kNoPivot | fix64::kOutOfRange;
+            }
+        }
+}
+
 // The panel's first 32 rows (mr of them exist), one warp, a row per lane: the 16 columns right-looking.
 // Leaves the diagonal block's entries in D, the pivots' reciprocal square roots in rsq, the entries
 // in W. Returns the number of columns factored (nb unless a pivot is not positive).
 template <int T>
-__device__ __forceinline__ int factor_diagonal(int k0, int mr, int nb, const int64_t* C, Limbs* W, int64_t ldw, Limbs* D,
+__device__ __forceinline__ int factor_diagonal(int k0, int mr, int nb, const int64_t* C, int64_t* W, int64_t ldw, Limbs* D,
                                                Rsqrt* rsq, unsigned char* bad) {
     using S = Shape<T>;
     int const lane = threadIdx.x & 31;
@@ -178,59 +331,68 @@ __device__ __forceinline__ int factor_diagonal(int k0, int mr, int nb, const int
     bool const no_pivot = mine && bad[k0 + lane] != 0;
     bool off = false;
     int done = nb;
+    // The next pivot's reciprocal square root is taken as soon as its column is up to date, beside the
+    // products of the columns after it.
+    int64_t t = acc[0] - fix64::total(0, cr[0]);
+    int64_t s = __shfl_sync(0xffffffffu, no_pivot ? (int64_t)-1 : t, 0);
+    if (s < fix64::kPivotMin) done = 0;
+    Rsqrt y = fix64::pivot_rsqrt(max(s, fix64::kPivotMin));
 #pragma unroll
     for (int j = 0; j < kNB; ++j) {
         if (j < done) {  // warp-uniform
-            int64_t const t = acc[j] - fix64::total(0, cr[j]);
-            int64_t const s = __shfl_sync(0xffffffffu, off || no_pivot ? (int64_t)-1 : t, j);
-            if (s < fix64::kPivotMin) {
-                done = j;
-            } else {
-                Rsqrt const y = fix64::pivot_rsqrt(s);
-                int64_t q;
-                bool const ok = fix64::scale_entry<fix64::kEntryBits>(t, y, q);
-                off |= !ok && lane > j;
-                Limbs const v = fix64::split(q);
-                if (lane >= j && mine) W[(k0 + lane) + (int64_t)(k0 + j) * ldw] = v;
-                if (lane < kNB) D[lane * kNB + j] = v;
-                if (lane == 0) rsq[j] = y;
+            int64_t q;
+            bool const ok = fix64::scale_entry<fix64::kEntryBits>(t, y, q);
+            off |= !ok && lane > j;
+            Limbs const v = fix64::split(q);
+            if (lane >= j && mine) W[(k0 + lane) + (int64_t)(k0 + j) * ldw] = S::kTensor ? fix64::to_digits(q) : fix64::pack(v);
+            if (lane < kNB) D[lane * kNB + j] = v;
+            if (lane == 0) rsq[j] = y;
 #pragma unroll
-                for (int c = j + 1; c < kNB; ++c) {
-                    int const h = __shfl_sync(0xffffffffu, v.h, c), l = __shfl_sync(0xffffffffu, v.l, c);
-                    fix64::mad(acc[c], -v.h, h);
-                    fix64::mad(cr[c], v.h, l);
-                    fix64::mad(cr[c], v.l, h);
+            for (int c = j + 1; c < kNB; ++c) {
+                int const h = __shfl_sync(0xffffffffu, v.h, c), l = __shfl_sync(0xffffffffu, v.l, c);
+                fix64::mad(acc[c], -v.h, h);
+                fix64::mad(cr[c], v.h, l);
+                fix64::mad(cr[c], v.l, h);
+                if (c == j + 1 && c < nb) {
+                    t = acc[c] - fix64::total(0, cr[c]);
+                    s = __shfl_sync(0xffffffffu, off || no_pivot ? (int64_t)-1 : t, c);
+                    if (s < fix64::kPivotMin) done = c;
+                    y = fix64::pivot_rsqrt(max(s, fix64::kPivotMin));
                 }
             }
         }
     }
+    // Pivots that were not reached: rows are still solved against the columns before them.
+    for (int j = done + lane; j < kNB; j += 32) rsq[j] = y;
     if (off) bad[k0 + lane] = fix64::kNoPivot | fix64::kOutOfRange;
     return done;
 }
 
-// Row r of the chunk against the diagonal block (its first `done` columns), one thread.
+// Row r of the chunk against the diagonal block, one thread. The columns past the first `done` are computed
+// from whatever D holds there, so that nothing branches between the columns, and not stored.
 template <int T>
-__device__ __forceinline__ void solve_row(int row, int r, int k0, int done, const int64_t* C, Limbs* W, int64_t ldw,
+__device__ __forceinline__ void solve_row(int row, int r, int k0, int done, const int64_t* C, int64_t* W, int64_t ldw,
                                           const Limbs* D, const Rsqrt* rsq, unsigned char* bad) {
     using S = Shape<T>;
     Limbs x[kNB];
     bool ok = true;
 #pragma unroll
     for (int j = 0; j < kNB; ++j) {
-        if (j < done) {
-            int64_t hh = 0, c0 = fix64::kCrossStart, c1 = 0;
+        int64_t hh = 0, c0 = fix64::kCrossStart, c1 = 0;
 #pragma unroll
-            for (int q = 0; q < j; ++q) {
-                Limbs const d = D[j * kNB + q];
-                fix64::mad(hh, x[q].h, d.h);
-                fix64::mad(c0, x[q].h, d.l);
-                fix64::mad(c1, x[q].l, d.h);
-            }
-            int64_t const t = C[j * S::CS + r] - fix64::total(hh, c0 + c1);
-            int64_t v;
-            ok &= fix64::scale_entry<fix64::kEntryBits>(t, rsq[j], v);
-            x[j] = fix64::split(v);
-            W[row + (int64_t)(k0 + j) * ldw] = x[j];
+        for (int q = 0; q < j; ++q) {
+            Limbs const d = D[j * kNB + q];
+            fix64::mad(hh, x[q].h, d.h);
+            fix64::mad(c0, x[q].h, d.l);
+            fix64::mad(c1, x[q].l, d.h);
+        }
+        int64_t const t = C[j * S::CS + r] - fix64::total(hh, c0 + c1);
+        int64_t v;
+        bool const in = fix64::scale_entry<fix64::kEntryBits>(t, rsq[j], v);
+        x[j] = fix64::split(v);
+        if (j < done) {
+            ok &= in;
+            W[row + (int64_t)(k0 + j) * ldw] = S::kTensor ? fix64::to_digits(v) : fix64::pack(x[j]);
         }
     }
     if (!ok) bad[row] = fix64::kNoPivot | fix64::kOutOfRange;
@@ -251,10 +413,11 @@ struct FixItem {
 };
 
 template <int T, class Batch>
-__global__ void __launch_bounds__(T, 512 / T) potrf_fix_kernel(Batch batch, int32_t* info) {
+__global__ void __launch_bounds__(T, T == 128 ? 3 : 512 / T) potrf_fix_kernel(Batch batch, int32_t* info) {
     using S = Shape<T>;
     extern __shared__ __align__(16) unsigned char smem[];
-    Limbs* stage = reinterpret_cast<Limbs*>(smem + S::kStage);
+    int64_t* stage = reinterpret_cast<int64_t*>(smem + S::kStage);
+    uint4* digits = reinterpret_cast<uint4*>(smem + S::kDigits);
     int64_t* C = reinterpret_cast<int64_t*>(smem + S::kChunk);
     Limbs* D = reinterpret_cast<Limbs*>(smem + S::kDiag);
     Rsqrt* rsq = reinterpret_cast<Rsqrt*>(smem + S::kRsqrt);
@@ -265,7 +428,7 @@ __global__ void __launch_bounds__(T, 512 / T) potrf_fix_kernel(Batch batch, int3
     FixItem it;
     if (!batch.get(b, it) || it.n > S::NMAX) return;
     int const n = it.n, tid = threadIdx.x;
-    Limbs* W = reinterpret_cast<Limbs*>(it.W);
+    int64_t* W = reinterpret_cast<int64_t*>(it.W);
     for (int i = tid; i < n; i += T) {
         int e;
         bad[i] = fix64::scale_exponent(it.A[i + (int64_t)i * it.lda], e) ? 0 : fix64::kNoPivot;
@@ -287,15 +450,19 @@ __global__ void __launch_bounds__(T, 512 / T) potrf_fix_kernel(Batch batch, int3
         int done = nb;
         for (int r0 = 0; r0 < m; r0 += T) {
             int const mr = min(T, m - r0);
+            if constexpr (S::kTensor) {
+                update_chunk_mma<T>(k0, r0, mr, nb, it.A, it.lda, W, it.ldw, stage, digits, C, scale, bad);
+            } else {
 #define BLASTGPU_UPDATE(RA) \
-    update_chunk<T, RA>(k0, r0, mr, nb, it.A, it.lda, W, it.ldw, stage, C, scale, bad)
-            switch ((mr + S::RT - 1) / S::RT) {
-                case 1: BLASTGPU_UPDATE(1); break;
-                case 2: BLASTGPU_UPDATE(2); break;
-                case 3: BLASTGPU_UPDATE(3); break;
-                default: BLASTGPU_UPDATE(4); break;
-            }
+    update_chunk_int<T, RA>(k0, r0, mr, nb, it.A, it.lda, W, it.ldw, stage, C, scale, bad)
+                switch ((mr + S::RT - 1) / S::RT) {
+                    case 1: BLASTGPU_UPDATE(1); break;
+                    case 2: BLASTGPU_UPDATE(2); break;
+                    case 3: BLASTGPU_UPDATE(3); break;
+                    default: BLASTGPU_UPDATE(4); break;
+                }
 #undef BLASTGPU_UPDATE
+            }
             cta_sync<T>();
             if (r0 == 0) {
                 if (tid < 32) {
@@ -320,20 +487,21 @@ __global__ void __launch_bounds__(T, 512 / T) potrf_fix_kernel(Batch batch, int3
     double const nan = __longlong_as_double(0x7ff8000000000000ll);
     int const lane = tid & 31, warp = tid >> 5;
     for (int c = warp; c < n; c += T / 32) {
-        Limbs const* w = W + (int64_t)c * it.ldw;
+        int64_t const* w = W + (int64_t)c * it.ldw;
         double* l = it.L + (int64_t)c * it.ldl;
         for (int i0 = c; i0 < n; i0 += 128) {
-            Limbs v[4];
+            int64_t v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 int const i = i0 + lane + 32 * u;
-                v[u] = i < n && c < good ? w[i] : Limbs{0, 0};
+                v[u] = i < n && c < good ? w[i] : 0;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 int const i = i0 + lane + 32 * u;
                 if (i < n) {
-                    double x = fix64::entry_to_double(fix64::join(v[u]), scale[i] - 61);
+                    int64_t const q = S::kTensor ? fix64::from_digits(v[u]) : fix64::join(fix64::unpack(v[u]));
+                    double x = fix64::entry_to_double(q, scale[i] - 61);
                     if (c >= good || (bad[i] & fix64::kOutOfRange)) x = nan;
                     l[i] = x;
                     if (it.L2) it.L2[i + (int64_t)c * it.ldl2] = x;
