@@ -370,3 +370,32 @@ def test_mixed_gesv_zero_pivot_reported(gpu):
     for i in (0, 2, 3):
         assert info[i] == 0 and berr[i] <= 1e-12
         assert _berr(As[i], B.to_list()[i], Bs[i]) <= 1.05e-12
+
+
+@pytest.mark.parametrize("n", [33, 64, 65, 66, 67, 68, 100, 127, 255, 256, 257])
+@pytest.mark.parametrize("nrhs,batch", [(1, 1), (4, 5), (5, 9), (3, 2000)])
+def test_getrs_backward_kernels_bitexact(gpu, oracle_lib, n, nrhs, batch):
+    """Sizes on both sides of the backward half's kernels, right-hand sides below, at and above the four that run
+    together, partial last warps, a batch too large for the shared-memory kernel: the oracle's bits."""
+    import torch
+
+    if batch == 2000 and n not in (65, 100, 257):
+        pytest.skip("one large batch per kernel is enough")
+    rng = np.random.default_rng(n * 10 + nrhs)
+    m = min(batch, 9)
+    LU, X = rng.standard_normal((m, n, n)) + 4 * np.eye(n), rng.standard_normal((m, n, nrhs))
+    piv = np.stack([rng.integers(k, n, m) for k in range(n)], axis=1).astype(np.int32)
+    rep = -(-batch // m)
+    dLU, dX = to_dev(np.tile(LU, (rep, 1, 1))[:batch], ld=n + 1), to_dev(np.tile(X, (rep, 1, 1))[:batch])
+    dp = torch.from_numpy(np.tile(piv, (rep, 1))[:batch]).cuda()
+    info = torch.zeros(batch, dtype=torch.int32, device="cuda")
+    if batch > 1:
+        info[1] = 3  # a singular factor: left alone
+    gpu.getrs(dLU, dp, dX, info)
+    torch.cuda.synchronize()
+    out = dX.cpu().numpy()
+    for b in {0, 1, batch // 2, batch - 1} & set(range(batch)):
+        want = np.asfortranarray(X[b % m].copy())
+        if b != 1:
+            oracle_lib.getrs(np.asfortranarray(LU[b % m]), piv[b % m], want, want)
+        assert np.array_equal(out[b], want), b
