@@ -60,9 +60,9 @@ int launch_syrk_lower(int m, int k, int trans_a, double alpha, const double* A, 
 int launch_potrs_cta_strided(int n, int nrhs, double* L, int ldl, int64_t sl, const double* B, int ldb, int64_t sb,
                              double* X, int ldx, int64_t sx, int64_t batch, cudaStream_t s);
 
-// Square matrices with n > kFixMinN - 1 are factored in 64-bit fixed point (potrf_fix.cu); up to 16 rows the
-// whole matrix is one panel of it, and the kernels that run a matrix in a thread, a quad or a warp
-// keep the products in binary64.
+// Square matrices of kFixMinN rows and more are factored in 64-bit fixed point (potrf_fix.cu, posv_pair.cu), save
+// the uniform batches that one thread per matrix does sooner (fixed_point_wanted in potrf.cu); up to 16 rows the
+// whole matrix is one block of it, and the products stay in binary64.
 constexpr int kFixMinN = 17;
 // L := chol(A), uniform batch, n <= 512. W: 8 bytes per entry of scratch with leading dimension ldw (nullptr: L
 // itself); L2: a second copy of the factor (nullptr: none). L may equal A, L2 may equal W.

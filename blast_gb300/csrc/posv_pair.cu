@@ -88,16 +88,17 @@ __device__ __forceinline__ void product_step(int64_t (&hh)[RA][4], int64_t (&cr)
 }
 
 // Block (I, J) of the matrix: binary64 entries to the remainders A - L L^T over the block columns
-// before J.
+// before J, for the block's first 4 RA rows.
+template <int RA>
 __device__ __forceinline__ void block_remainder(int64_t* P, int n, int I, int J, const int* scale, unsigned char* bad,
                                                 int rt, int ct) {
     int64_t* blk = P + block_at(I, J) + 4 * ct * kS + rt;
-    int64_t hh[4][4], cr[4][4];
+    int64_t hh[RA][4], cr[RA][4];
     int ec[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) ec[j] = scale[kB * J + 4 * ct + j];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < RA; ++i) {
         int const row = kB * I + rt + 4 * i, er = scale[row];
         int const cols = row < n ? row - kB * J - 4 * ct : -1;  // columns 0 .. cols of this lane's four exist
         bool ok = true;
@@ -116,24 +117,24 @@ __device__ __forceinline__ void block_remainder(int64_t* P, int n, int I, int J,
         int64_t const* cols = P + block_at(J, K) + 4 * ct;
 #pragma unroll 4
         for (int k = 0; k < kB; ++k) {
-            Limbs v[4], w[4];
+            Limbs v[RA], w[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = fix64::unpack(rows[4 * i]);
+            for (int i = 0; i < RA; ++i) v[i] = fix64::unpack(rows[4 * i]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) w[j] = fix64::unpack(cols[j]);
-            product_step<4>(hh, cr, v, w);
+            product_step<RA>(hh, cr, v, w);
             rows += kS;
             cols += kS;
         }
         if ((K & 1) != 0) {  // fix64::kFold terms since the last time
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RA; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) fix64::fold(hh[i][j], cr[i][j]);
         }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RA; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) blk[j * kS + 4 * i] = -fix64::total(hh[i][j], cr[i][j]);
 }
@@ -147,7 +148,7 @@ __device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int col
     int64_t acc[kB], cr[kB];
 #pragma unroll
     for (int c = 0; c < kB; ++c) {
-        acc[c] = blk[c * kS];
+        acc[c] = l16 < cols ? blk[c * kS] : 0;
         cr[c] = -fix64::kCrossStart;
     }
     bool const no_pivot = bad[l16] != 0;
@@ -189,8 +190,8 @@ __device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int col
     if (off) bad[l16] = fix64::kNoPivot | fix64::kOutOfRange;
 }
 
-// A row (this lane's, at row) against the diagonal block D.
-__device__ __forceinline__ bool solve_block_row(int64_t* row, const int64_t* D, const Rsqrt* rsq) {
+// A row (this lane's, at row) against the diagonal block D; mine: the row exists (else it becomes zeros).
+__device__ __forceinline__ bool solve_block_row(int64_t* row, bool mine, const int64_t* D, const Rsqrt* rsq) {
     Limbs x[kB];
     bool ok = true;
 #pragma unroll
@@ -204,7 +205,7 @@ __device__ __forceinline__ bool solve_block_row(int64_t* row, const int64_t* D, 
             fix64::mad(c1, x[q].l, d.h);
         }
         int64_t v;
-        ok &= fix64::scale_entry<fix64::kEntryBits>(row[j * kS] - fix64::total(hh, c0 + c1), rsq[j], v);
+        ok &= fix64::scale_entry<fix64::kEntryBits>((mine ? row[j * kS] : 0) - fix64::total(hh, c0 + c1), rsq[j], v);
         x[j] = fix64::split(v);
         row[j * kS] = fix64::pack(x[j]);
     }
@@ -263,7 +264,7 @@ __device__ __forceinline__ void rhs_remainder(const int64_t* P, int64_t* Y, cons
 // One right-hand side of block J (its remainders at y, units of 2^(ez - 62)) against the diagonal block:
 // the solution's limbs in place. Returns its exponent.
 template <bool BACK>
-__device__ __forceinline__ int solve_rhs_block(const int64_t* D, const Rsqrt* rsq, int64_t* y, int ez) {
+__device__ __forceinline__ int solve_rhs_block(const int64_t* D, const Rsqrt* rsq, int64_t* y, int ez, int cols) {
     constexpr int kBits = BACK ? kBwdBits : kFwdBits;
     int64_t top = 0;
 #pragma unroll
@@ -279,6 +280,8 @@ __device__ __forceinline__ int solve_rhs_block(const int64_t* D, const Rsqrt* rs
 #pragma unroll
         for (int k = 0; k < kB; ++k) {
             int const j = BACK ? kB - 1 - k : k;
+            x[j] = Limbs{0, 0};
+            if (j >= cols) continue;  // uniform in the warp
             int64_t hh = 0, c0 = fix64::kCrossStart, c1 = 0;
 #pragma unroll
             for (int m = 0; m < k; ++m) {
@@ -304,7 +307,7 @@ __device__ __forceinline__ int solve_rhs_block(const int64_t* D, const Rsqrt* rs
 
 // X(:, g0 .. g0 + nr - 1) of one matrix (16 lanes; the other matrix of the warp runs the same steps).
 template <int RA>
-__device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, int N, int blocks, int n, bool good, const int64_t* P,
+__device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, int N, int blocks, int nmax, int n, bool good, const int64_t* P,
                                             const Rsqrt* rsq, const int* scale, int64_t* Y, int* expo, int l16) {
     int const rt = l16 & 3, ct = l16 >> 2;
     bool const mine = l16 < nr;  // this lane's right-hand side
@@ -313,6 +316,7 @@ __device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, 
     bool finite = true;
     for (int J = 0; J < blocks; ++J) {
         int64_t* y = Y + J * kB * kGroup;
+        int const cols = min(kB, nmax - kB * J);
         int ez = 0;
         if (l16 < kGroup) {
             double b[kB];
@@ -344,7 +348,7 @@ __device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, 
             __syncwarp();
         }
         if (l16 < kGroup) {
-            int const e = solve_rhs_block<false>(P + block_at(J, J), rsq + kB * J, y + r, ez);
+            int const e = solve_rhs_block<false>(P + block_at(J, J), rsq + kB * J, y + r, ez, cols);
             expo[J * kGroup + r] = e;
             top = max(top, e);
         }
@@ -353,6 +357,7 @@ __device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, 
     top = -100000;
     for (int J = blocks - 1; J >= 0; --J) {
         int64_t* y = Y + J * kB * kGroup;
+        int const cols = min(kB, nmax - kB * J);
         int ez = 0;
         if (l16 < kGroup) {
             int const ey = expo[J * kGroup + r];
@@ -368,7 +373,7 @@ __device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, 
             __syncwarp();
         }
         if (l16 < kGroup) {
-            int const e = solve_rhs_block<true>(P + block_at(J, J), rsq + kB * J, y + r, ez);
+            int const e = solve_rhs_block<true>(P + block_at(J, J), rsq + kB * J, y + r, ez, cols);
             expo[J * kGroup + r] = e;
             top = max(top, e);
         }
@@ -453,12 +458,17 @@ __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t 
     __syncwarp();
     int fail = n;
     for (int J = 0; J < blocks; ++J) {
-        for (int I = J; I < blocks; ++I) block_remainder(P, n, I, J, scale, bad, l16 & 3, l16 >> 2);
+        for (int I = J; I < blocks; ++I) {
+            int const rows = nmax - kB * I;  // only the last block can have fewer than 16
+            if (rows <= 4) block_remainder<1>(P, n, I, J, scale, bad, l16 & 3, l16 >> 2);
+            else if (rows <= 8) block_remainder<2>(P, n, I, J, scale, bad, l16 & 3, l16 >> 2);
+            else block_remainder<4>(P, n, I, J, scale, bad, l16 & 3, l16 >> 2);
+        }
         __syncwarp();
         factor_diagonal(P + block_at(J, J), kB * J, min(kB, nmax - kB * J), rsq + kB * J, bad + kB * J, l16, fail);
         __syncwarp();
         for (int I = J + 1; I < blocks; ++I)
-            if (!solve_block_row(P + block_at(I, J) + l16, P + block_at(J, J), rsq + kB * J)) bad[kB * I + l16] = fix64::kNoPivot | fix64::kOutOfRange;
+            if (!solve_block_row(P + block_at(I, J) + l16, kB * I + l16 < nmax, P + block_at(J, J), rsq + kB * J)) bad[kB * I + l16] = fix64::kNoPivot | fix64::kOutOfRange;
         __syncwarp();
     }
     if (info && l16 == 0 && have) info[b] = fail < n ? fail + 1 : 0;
@@ -487,8 +497,8 @@ __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t 
         int const most = max(nrhs, __shfl_xor_sync(0xffffffffu, nrhs, 16));
         for (int g0 = 0; g0 < most; g0 += kGroup) {
             int const nr = max(0, min(kGroup, nrhs - g0));
-            if (min(kGroup, most - g0) <= 4) solve_group<1>(it, g0, nr, N, blocks, n, fail == n, P, rsq, scale, Y, expo, l16);
-            else solve_group<2>(it, g0, nr, N, blocks, n, fail == n, P, rsq, scale, Y, expo, l16);
+            if (min(kGroup, most - g0) <= 4) solve_group<1>(it, g0, nr, N, blocks, nmax, n, fail == n, P, rsq, scale, Y, expo, l16);
+            else solve_group<2>(it, g0, nr, N, blocks, nmax, n, fail == n, P, rsq, scale, Y, expo, l16);
         }
     }
 }

@@ -682,6 +682,19 @@ bool posv_quad_wanted(PosvArgs const& p) {
     return p.batch * 100 < (int64_t)t * 32 * 4 * sms;
 }
 
+// Whether a uniform batch is factored in fixed point. That cost goes by the size rounded up to 16, and a
+// warp's worth of matrices needs few warps; the thread-per-matrix kernel's goes by the size, and it needs a
+// batch that gives every scheduler two full warps. Measured on GB300 (binary64 against fixed point, us, 8
+// right-hand sides): n = 17 x 3,000: 92, 59; x 50,000: 537, 813. n = 20 x 10,000: 186, 171, the factor alone 78, 85.
+// n = 24 x 50,000: 963, 931, the factor alone 371, 415. n = 33 x 10,000: 534, 515; x 50,000: 1,954, 2,391. n = 40 x
+// 50,000: 2,689, 2,649. n = 52 x 50,000: 4,957, 5,530. Above 64 the fixed-point factor has a CTA to a matrix: n = 65
+// x 3,000: 1,370, 1,127; x 6,000: 1,556, 1,678; n = 76 x 10,000: 2,938, 2,746.
+bool fixed_point_wanted(int n, int64_t batch) {
+    if (n < kFixMinN || n > 512) return false;
+    if (batch >= 40000 && (n < 25 || (n <= 64 && (n & 15) >= 1 && (n & 15) <= 5))) return false;
+    return batch < 5000 || (n > 20 && (n <= 64 || n > 72));
+}
+
 int launch_posv(PosvArgs const& p, cudaStream_t stream) {
     if (p.batch == 0 || p.n == 0) {
         if (p.info && p.batch > 0 && p.mode != 2) {
@@ -690,8 +703,7 @@ int launch_posv(PosvArgs const& p, cudaStream_t stream) {
         }
         return BLASTGPU_SUCCESS;
     }
-    // Square matrices of kFixMinN rows and more are factored in fixed point; the solves follow.
-    if ((p.m == 0 || p.m == p.n) && p.mode != 2 && p.n >= kFixMinN && p.n <= 512) {
+    if ((p.m == 0 || p.m == p.n) && p.mode != 2 && fixed_point_wanted(p.n, p.batch)) {
         if (p.n <= kPairMaxN)
             return launch_posv_pair(p.n, p.mode == 1 ? p.nrhs : 0, p.A, p.lda, p.sa, p.L, p.ldl, p.sl, p.B, p.ldb, p.sb,
                                     p.X, p.ldx, p.sx, p.info, p.batch, stream);
@@ -851,7 +863,7 @@ int blastgpu_dposv_mirror_strided(int n, int nrhs, const double* A, int lda, int
     PosvArgs const p{n, nrhs, A, lda, stride_a, L_work, n, (int64_t)n * n, B, ldb, stride_b, X_work, n,
                      (int64_t)n * nrhs, info, batch, 1};
     MirrorOut const o{L, ldl, stride_l, X, ldx, stride_x};
-    if (n < kFixMinN || n > 512) {
+    if (!fixed_point_wanted(n, batch)) {
         posv_mirror_kernel<true><<<(unsigned)blocks, 32, 0, s>>>(p, o);
         return check_launch();
     }
