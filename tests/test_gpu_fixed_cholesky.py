@@ -153,3 +153,37 @@ def test_ragged_factor_is_the_uniform_one(gpu, ns):
         torch.cuda.synchronize()
         assert np.array_equal(np.tril(Lg), np.tril(P.cpu().numpy()[0])), n
         assert normwise(Xg, np.linalg.solve(Ah, Bh)) <= 100 * n * EPS, n
+
+
+@pytest.mark.parametrize("ns", [[3], [128, 1, 97, 0, 5, 66, 33], [65, 64, 63, 32, 31, 4, 2, 1], [127, 126, 125, 8, 100, 7, 0, 0, 16]])
+def test_ragged_solves_share_a_warp(gpu, ns):
+    """The backward substitutions of up to eight instances run in one warp: full and partial groups, sizes
+    of all remainders by 4, instances without rows, and instances with no or several right-hand sides."""
+    import torch
+
+    from blast_gb300.autograd import spd_solve_packed
+    from blast_gb300.ragged import Packed, PosvPlan
+
+    rng = np.random.default_rng(sum(ns) + len(ns))
+    rs = [(3 * i + 1) % 5 for i in range(len(ns))]
+    As = [spd(rng, n) for n in ns]
+    Bs = [rng.standard_normal((n, r)) for n, r in zip(ns, rs)]
+    A, B, X, L = Packed(ns, ns, "cuda"), Packed(ns, rs, "cuda"), Packed(ns, rs, "cuda"), Packed(ns, ns, "cuda")
+    A.fill_from(As)
+    B.fill_from(Bs)
+    plan = PosvPlan(A, B, X, L)
+    plan.run()
+    torch.cuda.synchronize()
+    assert not plan.results()[0].any()
+    a = A.buf.clone().requires_grad_()
+    b = B.buf.clone().requires_grad_()
+    x = spd_solve_packed(a, b, np.array(ns), np.array(rs))
+    x.sum().backward()
+    ga, gb, oa, ob = a.grad.cpu().numpy(), b.grad.cpu().numpy(), 0, 0
+    for n, r, Ah, Bh, Xg in zip(ns, rs, As, Bs, X.to_list()):
+        if n * r:
+            want, g = np.linalg.solve(Ah, Bh), np.linalg.solve(Ah, np.ones((n, r)))
+            assert normwise(Xg, want) <= 100 * n * EPS, n
+            assert normwise(gb[ob:ob + n * r].reshape((n, r), order="F"), g) <= 100 * n * EPS, n
+            assert normwise(ga[oa:oa + n * n].reshape((n, n), order="F"), -0.5 * (g @ want.T + want @ g.T)) <= 200 * n * EPS, n
+        oa, ob = oa + n * n, ob + n * r
