@@ -73,12 +73,13 @@ int launch_potrf_fix(const blastgpu_posv_desc* desc, int min_n, int max_n, int32
 int launch_potrf_fix(const blastgpu_posv_bwd_desc* desc, int min_n, int max_n, int32_t* info, int64_t batch,
                      cudaStream_t s);
 
-// Factorisation and, with nrhs > 0, solve in fixed point, two matrices per warp (posv_pair.cu), n <= 64. L may
+// Factorisation and, with nrhs > 0, solve in fixed point, two matrices per warp (posv_pair.cu), n <= 64. host: the
+// operands are in host memory, which changes the order of loads and stores and no result. L may
 // equal A, X may equal B.
 constexpr int kPairMaxN = 64;
 int launch_posv_pair(int n, int nrhs, const double* A, int lda, int64_t sa, double* L, int ldl, int64_t sl,
                      const double* B, int ldb, int64_t sb, double* X, int ldx, int64_t sx, int32_t* info, int64_t batch,
-                     cudaStream_t s);
+                     bool host, cudaStream_t s);
 // Ragged: the instances with A and min_n <= rows <= max_n.
 int launch_posv_pair(const blastgpu_posv_desc* desc, int min_n, int max_n, int32_t* info, int64_t batch, cudaStream_t s);
 

@@ -8,9 +8,9 @@
 // quarter of them the products of block columns, and the chain of pivots, with 8 warps per SM. 50,000
 // matrices of n = 48 with 8 right-hand sides take 3.11 ms (1.24 ms the factor alone) against 4.15 ms for
 // a binary64 thread per matrix, which the binary64 pipe holds at 3.0 ms at best; 10,000 take a half, one
-// matrix of n = 24 23 us a call instead of 53. A
-// matrix has 16 lanes, so that the work on the diagonal, which has 16 rows to share it, fills the warp
-// with two matrices, and a batch of small matrices needs few warps. The matrix is read from memory
+// matrix of n = 24 21 us a call instead of 53. A matrix has 16 lanes, so that the work on the diagonal,
+// which has 16 rows to share it, fills the warp with two matrices, and a batch of small matrices needs few
+// warps. The matrix is read from memory
 // once and written once; the earlier columns, which a thread per matrix reads again for every strip,
 // stay in shared memory.
 //
@@ -397,7 +397,28 @@ __device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, 
     __syncwarp();
 }
 
-template <bool SOLVE, class Batch>
+// Operands in host memory (HOST): the link to it carries lines of 16 entries, and its memory is read and written
+// fastest along one stretch. So the columns are read one after another, each in whole lines, and a block column of the
+// factor goes out as soon as it is there, with the other direction still busy. 50,000 matrices of n = 48 with 8
+// right-hand sides take 4.91 ms with three batches in flight and 5.11 alone (row blocks of A read, and L written,
+// at once: 5.25, 5.50), 10,000 1.18 ms (1.29), 30,000 of n = 60 5.2 (5.6); prefetches into L2 gave nothing.
+// Columns kB J .. kB J + 15 of the factor:
+__device__ __forceinline__ void store_columns(PairItem const& it, int n, int J, int blocks, int fail, const int64_t* P,
+                                              const int* scale, const unsigned char* bad, int l16) {
+    for (int col = kB * J; col < min(n, kB * J + kB); ++col) {
+        double* l = it.L + (int64_t)col * it.ldl;
+        int const at = (int)(reinterpret_cast<uintptr_t>(l) >> 3) & 15;
+        for (int r = col - ((col + at) & 15) + l16; r < n; r += kB) {
+            if (r < col) continue;
+            double const x = fix64::entry_to_double(
+                fix64::join(fix64::unpack(P[block_at(r / kB, J) + col % kB * kS + r % kB])), scale[r] - 61);
+            int const first_nan = (bad[r] & fix64::kOutOfRange) ? 0 : fail;
+            l[r] = col >= first_nan ? __longlong_as_double(0x7ff8000000000000ll) : x;
+        }
+    }
+}
+
+template <bool SOLVE, bool HOST, class Batch>
 __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t count, int N, int32_t* info) {
     extern __shared__ __align__(16) unsigned char smem[];
     int const l16 = threadIdx.x & 15, half = threadIdx.x >> 4;
@@ -418,17 +439,30 @@ __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t 
     if (nmax == 0) return;
     int const blocks = (nmax + kB - 1) / kB;  // the warp's; the layout stays that of N
     // lower(A) to shared memory, all loads in flight together
-    for (int I = 0; I < blocks; ++I) {
-        int const r = kB * I + l16;
-        if (r < n) {
-            for (int J = 0; J <= I; ++J) {
-                unsigned const d = (unsigned)__cvta_generic_to_shared(P + block_at(I, J) + l16);
-                double const* a = it.A + r + (int64_t)(kB * J) * it.lda;
+    if constexpr (HOST) {
+#pragma unroll 2
+        for (int j = 0; j < n; ++j) {
+            double const* a = it.A + (int64_t)j * it.lda;
+            int const at = (int)(reinterpret_cast<uintptr_t>(a) >> 3) & 15;
+            for (int r = j - ((j + at) & 15) + l16; r < n; r += kB)
+                if (r >= j)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(
+                                     P + block_at(r / kB, j / kB) + j % kB * kS + r % kB)), "l"(a + r)
+                                 : "memory");
+        }
+    } else {
+        for (int I = 0; I < blocks; ++I) {
+            int const r = kB * I + l16;
+            if (r < n) {
+                for (int J = 0; J <= I; ++J) {
+                    unsigned const d = (unsigned)__cvta_generic_to_shared(P + block_at(I, J) + l16);
+                    double const* a = it.A + r + (int64_t)(kB * J) * it.lda;
 #pragma unroll 4
-                for (int c = 0; c < kB; ++c)
-                    if (kB * J + c <= r)
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d + 8 * c * kS), "l"(a + c * it.lda)
-                                     : "memory");
+                    for (int c = 0; c < kB; ++c)
+                        if (kB * J + c <= r)
+                            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d + 8 * c * kS), "l"(a + c * it.lda)
+                                         : "memory");
+                }
             }
         }
     }
@@ -470,11 +504,16 @@ __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t 
         for (int I = J + 1; I < blocks; ++I)
             if (!solve_block_row(P + block_at(I, J) + l16, kB * I + l16 < nmax, P + block_at(J, J), rsq + kB * J)) bad[kB * I + l16] = fix64::kNoPivot | fix64::kOutOfRange;
         __syncwarp();
+        if constexpr (HOST) store_columns(it, n, J, blocks, fail, P, scale, bad, l16);
     }
     if (info && l16 == 0 && have) info[b] = fail < n ? fail + 1 : 0;
     // The factor to memory. After a pivot that is not positive the columns from it on are NaN, and so are
     // the rows whose entries left the fixed-point range.
-    for (int I = 0; I < blocks; ++I) {
+    bool again = !HOST;  // in host memory already, but for rows found out of range since
+    if constexpr (HOST)
+        for (int i = l16; i < n; i += kB) again |= (bad[i] & fix64::kOutOfRange) != 0;
+    again = __any_sync(0xffffffffu, again);
+    for (int I = 0; I < (again ? blocks : 0); ++I) {
         int const r = kB * I + l16, e = scale[r] - 61, first_nan = (bad[r] & fix64::kOutOfRange) ? 0 : fail;
         if (r < n) {
             for (int J = 0; J <= I; ++J) {
@@ -525,15 +564,15 @@ struct PairDesc {
     }
 };
 
-template <bool SOLVE, class Batch>
+template <bool SOLVE, bool HOST = false, class Batch>
 int launch(Batch const& batch, int max_n, int64_t count, int32_t* info, cudaStream_t s) {
     if (count == 0) return BLASTGPU_SUCCESS;
     if (max_n > kMaxN || (count + 1) / 2 > 0x7fffffff) return BLASTGPU_ERR_TOO_LARGE;
     int const N = (max_n + kB - 1) / kB;
     size_t const smem = 2 * (size_t)layout_of(N, SOLVE).bytes;
-    cudaError_t const e = ensure_smem<posv_pair_kernel<SOLVE, Batch>>(2 * (size_t)layout_of(kMaxN / kB, SOLVE).bytes);
+    cudaError_t const e = ensure_smem<posv_pair_kernel<SOLVE, HOST, Batch>>(2 * (size_t)layout_of(kMaxN / kB, SOLVE).bytes);
     if (e != cudaSuccess) { set_cuda_error(e); return BLASTGPU_ERR_CUDA; }
-    posv_pair_kernel<SOLVE, Batch><<<(unsigned)((count + 1) / 2), 32, smem, s>>>(batch, count, N, info);
+    posv_pair_kernel<SOLVE, HOST, Batch><<<(unsigned)((count + 1) / 2), 32, smem, s>>>(batch, count, N, info);
     return check_launch();
 }
 
@@ -541,8 +580,9 @@ int launch(Batch const& batch, int max_n, int64_t count, int32_t* info, cudaStre
 
 int launch_posv_pair(int n, int nrhs, const double* A, int lda, int64_t sa, double* L, int ldl, int64_t sl,
                      const double* B, int ldb, int64_t sb, double* X, int ldx, int64_t sx, int32_t* info, int64_t batch,
-                     cudaStream_t s) {
+                     bool host, cudaStream_t s) {
     PairStrided const p{n, nrhs, A, lda, sa, L, ldl, sl, nrhs ? B : nullptr, ldb, sb, nrhs ? X : nullptr, ldx, sx};
+    if (host) return nrhs ? launch<true, true>(p, n, batch, info, s) : launch<false, true>(p, n, batch, info, s);
     return nrhs ? launch<true>(p, n, batch, info, s) : launch<false>(p, n, batch, info, s);
 }
 

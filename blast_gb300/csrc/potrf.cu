@@ -1,4 +1,6 @@
-// Batched Cholesky factorisation and solve (potrf, potrs, posv), binary64, sm_103a.
+// Batched Cholesky factorisation and solve (potrf, potrs, posv): the entry points, and the binary64
+// kernels with a thread or a quad of lanes per matrix, sm_103a. Most square batches of 17 <= n <= 512
+// are factored by posv_pair.cu and potrf_fix.cu instead (fixed_point_wanted).
 //
 // Reference: blast::potrf (dense/Potrf.hpp:20-106): left-looking, column strips of KN = 4,
 // each strip covered top-down by register tiles of 12, 8 and 4 rows (TileSize<double> = 4).
@@ -706,7 +708,7 @@ int launch_posv(PosvArgs const& p, cudaStream_t stream) {
     if ((p.m == 0 || p.m == p.n) && p.mode != 2 && fixed_point_wanted(p.n, p.batch)) {
         if (p.n <= kPairMaxN)
             return launch_posv_pair(p.n, p.mode == 1 ? p.nrhs : 0, p.A, p.lda, p.sa, p.L, p.ldl, p.sl, p.B, p.ldb, p.sb,
-                                    p.X, p.ldx, p.sx, p.info, p.batch, stream);
+                                    p.X, p.ldx, p.sx, p.info, p.batch, false, stream);
         int const st = launch_potrf_fix(p.n, p.A, p.lda, p.sa, p.L, p.ldl, p.sl, nullptr, 0, 0, nullptr, 0, 0, p.info,
                                         p.batch, stream);
         if (st != BLASTGPU_SUCCESS || p.mode == 0 || p.nrhs == 0) return st;
@@ -869,7 +871,7 @@ int blastgpu_dposv_mirror_strided(int n, int nrhs, const double* A, int lda, int
     }
     if (n <= kPairMaxN)  // the working copy is shared memory
         return launch_posv_pair(n, nrhs, A, lda, stride_a, L, ldl, stride_l, B, ldb, stride_b, X, ldx, stride_x, info,
-                                batch, s);
+                                batch, true, s);
     int const st = launch_potrf_fix(n, A, lda, stride_a, L, ldl, stride_l, L_work, n, (int64_t)n * n, L_work, n,
                                     (int64_t)n * n, info, batch, s);
     if (st != BLASTGPU_SUCCESS || nrhs == 0) return st;

@@ -187,3 +187,37 @@ def test_ragged_solves_share_a_warp(gpu, ns):
             assert normwise(gb[ob:ob + n * r].reshape((n, r), order="F"), g) <= 100 * n * EPS, n
             assert normwise(ga[oa:oa + n * n].reshape((n, n), order="F"), -0.5 * (g @ want.T + want @ g.T)) <= 200 * n * EPS, n
         oa, ob = oa + n * n, ob + n * r
+
+
+@pytest.mark.parametrize("n", [17, 24, 40, 48, 60, 61, 64])
+@pytest.mark.parametrize("nrhs", [0, 3])
+def test_host_order_is_the_device_order(gpu, n, nrhs):
+    """The entry for operands in host memory reads and writes in another order: same bits, at leading
+    dimensions that put the columns off the lines, with a pivot that is not positive, NaN and infinity."""
+    import torch
+
+    from blast_gb300 import _lib
+
+    rng = np.random.default_rng(n + nrhs)
+    A = spd_batch(rng, 5, n)
+    A[1, n // 2, n // 2] = -1.0
+    A[2, n - 1, 3] = np.nan
+    A[3, n - 2, 1] = np.inf
+    ld = n + 3
+    dA, dB = to_dev(A, ld=ld), to_dev(rng.standard_normal((5, n, max(nrhs, 1))), ld=ld)
+    L, X = gpu.col_major((5,), n, n, "cuda").zero_(), gpu.col_major((5,), n, max(nrhs, 1), "cuda").zero_()
+    info = gpu.posv(dA, L, dB, X) if nrhs else gpu.potrf(dA, L)
+    hL, hX = torch.zeros(5 * ld * n).double().pin_memory(), torch.zeros(5 * ld * n).double().pin_memory()
+    wL, wX = torch.empty(5 * n * n, device="cuda").double(), torch.empty(5 * n * n, device="cuda").double()
+    hinfo = torch.zeros(5, dtype=torch.int32, device="cuda")
+    _lib.call("blastgpu_dposv_mirror_strided", n, nrhs, dA.data_ptr(), ld, dA.stride(0), dB.data_ptr(), ld,
+              dB.stride(0), hL.data_ptr(), ld, ld * n, hX.data_ptr(), ld, ld * n, wL.data_ptr(), wX.data_ptr(),
+              hinfo.data_ptr(), 5, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(hinfo, info.to(hinfo.dtype))
+    gotL = np.tril(hL.numpy().reshape(5, n, ld).transpose(0, 2, 1)[:, :n])
+    assert np.array_equal(gotL, np.tril(L.cpu().numpy()), equal_nan=True)
+    assert not hL.numpy().reshape(5, n, ld)[:, :, n:].any()
+    if nrhs:
+        gotX = hX.numpy().reshape(5, n, ld)[:, :nrhs].transpose(0, 2, 1)[:, :n]
+        assert np.array_equal(gotX, X.cpu().numpy(), equal_nan=True)
