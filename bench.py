@@ -12,8 +12,9 @@ with the oracle (BLAST's algorithm restated in C++) and with LAPACK on a strided
 
 Prints one JSON line. `value` is matrices/s measured with CUDA events on the launching stream
 (max over ranks); `e2e` is the same metric through the public API with pinned host buffers and
-the host<->device traffic inside the timed region; `roofline` is the binary64 issue bound of the
-dominant kernel; `cpu_baseline` times the CPU restatement of BLAST's algorithm on this host.
+the host<->device traffic inside the timed region; `roofline` sets it against the binary64 FMA peak (the
+dominant kernel multiplies in 64-bit fixed point on the integer pipe, so that peak is a yardstick, not
+its bound); `cpu_baseline` times the CPU restatement of BLAST's algorithm on this host.
 The keys `gemm24`, `lu_ragged`, `mixed_ir` and `adjoint` carry the other workloads (24x24 gemm
 batch, ragged LU, mixed precision + refinement, differentiable solve), each with its timing,
 roofline, CPU baseline and parity against the oracle and LAPACK on its own inputs.
@@ -440,7 +441,7 @@ def config_lu_ragged(steps: int, peak: float | None, count: int = 20_000, cpu: b
            "ms_per_step": ms, "matrices_per_s": count / ms * 1e3, "gflops": flops / ms / 1e6, "steps": steps,
            "timing_note": "each step re-copies the inputs (getrf works in place); the copy time, timed "
                           "alone, is subtracted",
-           "roofline": _roofline(flops, nbytes, ms, peak, "getrf_cta_kernel + getrf_warp_kernel + getrs_kernel"),
+           "roofline": _roofline(flops, nbytes, ms, peak, "getrf_cta_kernel + getrf_warp_kernel + getrs_bwd_kernel"),
            "parity": {"n_checked": count,
                       "pivot_sequences_identical_to_oracle": count - piv_mismatch,
                       "pivot_mismatches_vs_oracle": piv_mismatch,
@@ -697,8 +698,8 @@ def config_adjoint(steps: int, peak: float | None, count: int = 8192) -> dict:
     return {"workload": "differentiable SPD solve, 8,192 x n ~ U{32..128}, A = G G^T + n I, 1 RHS, seed 55",
             "forward_ms": ms_f, "backward_ms": ms_b, "steps": steps,
             "forward_matrices_per_s": count / ms_f * 1e3, "backward_matrices_per_s": count / ms_b * 1e3,
-            "forward_roofline": _roofline(f_flops, f_bytes, ms_f, peak, "posv_cta_f64_kernel"),
-            "backward_roofline": _roofline(b_flops, b_bytes, ms_b, peak, "posv_bwd_kernel"),
+            "forward_roofline": _roofline(f_flops, f_bytes, ms_f, peak, "potrf_fix_kernel + posv_pair_kernel + posv_warp_kernel"),
+            "backward_roofline": _roofline(b_flops, b_bytes, ms_b, peak, "posv_bwd_warp_kernel"),
             "parity": {"n_checked": int(len(idx)),
                        "x_max_normwise_vs_oracle": max(ex_o), "x_max_normwise_vs_lapack": max(ex_l),
                        "dL_db_max_normwise_vs_cpu_fp64": max(egb), "dL_dA_max_normwise_vs_cpu_fp64": max(ega),
@@ -711,8 +712,7 @@ def config_adjoint(steps: int, peak: float | None, count: int = 8192) -> dict:
 # ---------------------------------------------------------------------------------------------
 def workload_riccati(args):
     """BLAST's Riccati kernel (bench/blas/SyrkPotrf.cpp): D = chol(C + A^T*A), A 30 x 60, C 60 x 60
-    SPD, 50,000 instances; the fused kernel against the entry point's default, syrkLower followed
-    by potrf (two launches)."""
+    SPD, 50,000 instances, through the one entry point and as syrkLower followed by potrf."""
     import numpy as np
     import torch
 
@@ -732,13 +732,13 @@ def workload_riccati(args):
     C.copy_(G @ G.mT + n * torch.eye(n, device="cuda", dtype=torch.float64))
     del G
     D, S = bg.col_major((batch,), n, n, "cuda"), bg.col_major((batch,), n, n, "cuda")
-    from blast_gb300 import _lib
+    one = _timed(lambda: bg.syrk_potrf(1.0, A, 1.0, C, D), args.steps)
 
-    _lib.tune_set("syrk_potrf.fused_min_batch", 0)  # the fused kernel ...
-    fused = _timed(lambda: bg.syrk_potrf(1.0, A, 1.0, C, D), args.steps)
-    _lib.tune_set("syrk_potrf.fused_min_batch", 0x7FFFFFFF)  # ... and the entry point's default
+    def composed():
+        bg.syrk_lower(1.0, Acol, 1.0, C, S)
+        bg.potrf(S, S)
 
-    comp = _timed(lambda: bg.syrk_potrf(1.0, A, 1.0, C, S), args.steps)
+    comp = _timed(composed, args.steps)
     torch.cuda.synchronize()
     same = bool(torch.equal(torch.tril(D), torch.tril(S)))
     flops = n * (n + 1) * m + n ** 3 / 3 + n ** 2 / 2 + n / 6
@@ -755,8 +755,7 @@ def workload_riccati(args):
         done += len(hA)
     cpu = done / (time.perf_counter() - t0)
     return {"workload": f"syrk+potrf (Riccati) {batch} x D = chol(C + A^T A), A {m}x{n}",
-            "fused_ms": fused, "fused_matrices_per_s": batch / fused * 1e3,
-            "fused_tflops": flops * batch / fused / 1e9, "composed_ms": comp,
+            "ms": one, "matrices_per_s": batch / one * 1e3, "tflops": flops * batch / one / 1e9, "composed_ms": comp,
             "composed_matrices_per_s": batch / comp * 1e3, "bitwise_equal": same,
             "cpu_port_matrices_per_s_1thread": cpu}
 
@@ -766,42 +765,25 @@ def workload_riccati(args):
 # ---------------------------------------------------------------------------------------------
 def workload_posv_batches(args) -> dict:
     """Cholesky solves n = 48 with 8 right-hand sides (A = G G^T + 48 I, B ~ N(0,1)) at batch sizes
-    from 500 to 50,000: the library's launch choice (one thread per matrix, or a quad of lanes per
-    matrix for batches that hold fewer than 1.5 full warps per SM sub-partition) against the
-    thread-per-matrix kernel alone ("posv.quad" = 0), with the two results compared bit for bit."""
-    import numpy as np
+    from 500 to 50,000."""
     import torch
 
     import blast_gb300 as bg
-    from blast_gb300 import _lib
 
     dev = torch.device("cuda", 0)
-    key = "posv.quad.n64"
-    default = _lib.tune_get(key)
     rows = []
     for batch in (500, 2_000, 8_000, 16_000, 24_000, 50_000):
         A_h, B_h = host_inputs(batch, SEED)
         A, B = _to_dev_batch(A_h, dev), _to_dev_batch(B_h, dev)
         L = bg.col_major((batch,), N, N, dev)
         X = bg.col_major((batch,), N, NRHS, dev)
-        row = {"batch": batch}
-        outs = {}
-        for name, q in (("library", default), ("thread_kernel", 0)):
-            if q is None:
-                q = 150
-            _lib.tune_set(key, q)
-            row[f"{name}_ms"] = _timed(lambda: bg.posv(A, L, B, X), args.steps)
-            outs[name] = (L.cpu().numpy(), X.cpu().numpy())
-        _lib.tune_set(key, 150 if default is None else default)
-        row["speedup"] = row["thread_kernel_ms"] / row["library_ms"]
-        row["bit_identical"] = all(np.array_equal(a, b) for a, b in zip(outs["library"], outs["thread_kernel"]))
-        rows.append(row)
+        rows.append({"batch": batch, "ms": _timed(lambda: bg.posv(A, L, B, X), args.steps)})
         del A, B, L, X
     return {"workload": "posv n = 48, 8 RHS, batch 500 .. 50,000", "steps": args.steps, "rows": rows}
 
 
 def _traffic_from_profile(batch: int):
-    p = ROOT / "profiles" / "posv_thread_n48_traffic.json"
+    p = ROOT / "profiles" / "posv_pair_n48_traffic.json"
     try:
         t = json.loads(p.read_text())
     except (OSError, ValueError):
@@ -964,7 +946,7 @@ def run_ours(args):
                      "algorithmic_bytes": BATCH * BYTES_PER,
                      "peak_source": "binary64 FMA probe kernel run in this process (MEASURED_PEAKS.json has no FP64 figure)",
                      "peak_dmma_tflops": peak_dmma,
-                     "kernel": "posv_thread_kernel"},
+                     "kernel": "posv_pair_kernel"},
         "parity": parity,
         "e2e": {"value": ws * BATCH / (e2e_ms * 1e-3), "unit": "matrices/s",
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

@@ -137,7 +137,7 @@ def potrf(A: torch.Tensor, L: torch.Tensor) -> torch.Tensor:
 
 def posv(A: torch.Tensor, L: torch.Tensor, B: torch.Tensor, X: torch.Tensor) -> torch.Tensor:
     """Cholesky solve A*X = B: potrf(A, L), trsm<Lower>(L, B, X), trsm<Upper>(trans(L), X, X)
-    (dense/Potrf.hpp:66-106, dense/Trsm.hpp:17-66), fused in one launch. Returns info."""
+    (dense/Potrf.hpp:66-106, dense/Trsm.hpp:17-66). Returns info."""
     a, l, b, x = (_as_mat(t, n) for t, n in ((A, "A"), (L, "L"), (B, "B"), (X, "X")))
     n = a.rows
     if a.cols != n or l.rows != n or l.cols != n or b.rows != n or x.rows != n or x.cols != b.cols:
@@ -231,7 +231,7 @@ def syrk_lower(alpha, A: torch.Tensor, beta, C: torch.Tensor, D: torch.Tensor) -
 
 
 def syrk_potrf(alpha, A: torch.Tensor, beta, C: torch.Tensor, D: torch.Tensor) -> torch.Tensor:
-    """D = chol(beta*C + alpha*A*A^T), lower, fused (syrkLower then potrf: dense/Syrk.hpp:15-145,
+    """D = chol(beta*C + alpha*A*A^T), lower (syrkLower then potrf: dense/Syrk.hpp:15-145,
     dense/Potrf.hpp:66-106; BLAST's Riccati benchmark bench/blas/SyrkPotrf.cpp:15-40).
 
     A is n x k, column-major, or a row-major tensor (BLAST's trans() view: op(A) = A^T of a k x n

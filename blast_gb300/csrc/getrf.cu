@@ -18,9 +18,9 @@
 //    IEEE division, as in BLAST), so factors and pivot sequences are bit-identical to the oracle.
 //  * getrs: the forward half (laswp(b), unit-lower solve) one warp per matrix for n <= 256, lanes
 //    over rows in a column sweep that keeps every row's ascending order; the backward half one
-//    thread per matrix. The backward substitution is a chain of dependent dot products in BLAST's
-//    order (each x_i starts from x_{i+1}); running it per thread keeps every lane busy while
-//    preserving that order.
+//    thread per matrix, or four matrices per warp out of shared memory (getrs_bwd_kernel). The
+//    backward substitution is a chain of dependent dot products in BLAST's order (each x_i starts
+//    from x_{i+1}), so one thread follows it and its order is kept.
 #include <math_constants.h>
 
 #include <atomic>

@@ -1,5 +1,6 @@
-// Ragged batched Cholesky solve for medium sizes (one CTA per matrix), binary64 and
-// mixed precision (binary32 factorisation + binary64 iterative refinement), sm_103a.
+// Batched Cholesky solves for medium sizes, one CTA per matrix: mixed precision (binary32
+// factorisation + binary64 iterative refinement) and the binary64 substitutions with a factor that is
+// there already (from potrf_fix.cu or the caller), sm_103a.
 //
 // Reference: blast::potrf (dense/Potrf.hpp:66-106) is left-looking: each column strip is first
 // updated with all previous columns (the ger(-1, ...) loop, a gemm), then factored on the
@@ -7,7 +8,7 @@
 // (dense/Trsm.hpp:17-66). BLAST has no mixed precision and no refinement; that part is new.
 //
 // GPU mapping: one CTA of 256 threads (8 warps) per matrix, the whole solve in one launch.
-//  * Factorisation, left-looking with panels of 32 columns. Warp w owns panel columns
+//  * Factorisation (binary32), left-looking with panels of 32 columns. Warp w owns panel columns
 //    4w..4w+3, lane l owns rows l, l+32, ..., so each thread keeps an MAXR x 4 register tile
 //    (BLAST's RegisterMatrix, 32 times wider). The update of a panel with all previous columns
 //    streams those columns through shared memory with cp.async, 16 at a time and double-buffered
@@ -15,9 +16,9 @@
 //    fused multiply-adds per column (RA = 32-row blocks still below the diagonal, fixed at
 //    compile time per panel) with operands read conflict-free from shared memory (rows:
 //    consecutive lanes; panel columns: a warp-uniform broadcast).
-//  * The 32 x 32 diagonal block is factored in place in shared memory: binary64 column at a time
-//    by all threads with warp 0 finishing each pivot column, binary32 in sub-panels of 8 columns
-//    factored by warp 0 in registers. The rows below are then solved against it (one thread per
+//  * The 32 x 32 diagonal block is factored in place in shared memory, in sub-panels of 8 columns
+//    factored by warp 0 in registers (binary64 on request: column at a time by all threads with
+//    warp 0 finishing each pivot column). The rows below are then solved against it (one thread per
 //    row), and the panel is written to the factor.
 //  * Forward and backward substitution run blockwise with look-ahead: once a 32-row block is
 //    solved, warp 0 applies it to the next block and solves that block's triangle from registers
@@ -48,7 +49,7 @@ constexpr int kKC = 32;  // previous columns staged at once by the panel update,
 struct CtaItem {
     int n;
     const double* A; int lda;
-    double* L; int ldl;       // binary64 factor output (plain path) or nullptr
+    double* L; int ldl;       // the binary64 factor (plain solves) or nullptr
     const double* B; int ldb;
     double* X; int ldx;
     int nrhs;

@@ -9,14 +9,17 @@ as BLAST's do. Three transports:
   engines bring each chunk's results back while the next chunk computes. On GB300 the kernel's
   reads cross NVLink-C2C as it computes, so only the result direction is staged.
 * ``"mirror"``: one launch (blastgpu_dposv_mirror_strided); the kernel reads the host inputs
-  directly and each warp, once its 32 instances are solved, writes their L and X to the host
-  buffers with whole-line stores, while other warps compute. With ``depth`` > 1, up to ``depth``
+  directly and each warp writes its instances' L and X to the host buffers with whole-line stores
+  as soon as it has them, while other warps compute. With ``depth`` > 1, up to ``depth``
   batches are in flight at once, each on a stream and a device workspace of its own: the next
   batch's warps start reading their inputs over the host link while the previous batch's warps
   still compute, so the link and the binary64 pipes stay busy together (every warp of one launch
   asks for its next strip at about the same moment, which leaves the link idle while they compute).
 
 Device buffers are allocated once per pipeline and reused.
+
+L and X agree with a solve of the same batch in device memory to rounding, not always to the bit: for 17 <= n <= 64
+the kernel, and with it the rounding, follows from the size of the batch that one launch gets (a chunk here).
 """
 from __future__ import annotations
 

@@ -14,12 +14,12 @@ Tunable choices (read by the library through blastgpu_tune_set / tune_get_bin):
 * ``posv.mixed.n<bin>`` — ragged mixed-precision Cholesky factorisation per size bin (the modes of
   posv_cta_mixed_kernel); timed on the mixed workload's matrices (cond 1e2, 1e4, 1e6) and kept only
   if every instance converges.
-* ``posv.cta_min_n`` — uniform Cholesky batches from this n on run one CTA per matrix instead of one
-  thread per matrix.
-* ``posv.warp.n<bin>`` — ragged binary64 Cholesky batches with every n <= 128: one warp (1) or one
-  CTA (0) per matrix (same bits as the thread kernel, or within 10 n eps of it).
-* ``posv.quad.n<bin>`` — uniform Cholesky batches (thread-per-matrix sizes) run a quad of lanes per
-  matrix when they hold fewer than value / 100 full warps per SM sub-partition (same bits; not
+* ``posv.cta_min_n`` — uniform solves with a given factor from this n on run one CTA per matrix
+  instead of one thread per matrix.
+* ``posv.warp.n<bin>`` — ragged binary64 Cholesky solves with every n <= 128: the substitutions (and
+  for n <= 16 the factor) by one warp (1) or one CTA (0) per matrix (within 10 n eps of each other).
+* ``posv.quad.n<bin>`` — uniform Cholesky batches that run in binary64 on a thread per matrix run a
+  quad of lanes per matrix when they hold fewer than value / 100 full warps per SM sub-partition (same bits; not
   timed by this module: the library's defaults, 0 / 50 / 150 / 150 / 150 / 150 for the bins 8 to
   128, come from ``bench.py --workload posv_batches`` style measurements).
 

@@ -24,9 +24,11 @@
  *   BLASTGPU_PANEL      data[(i/ps)*ld + i%ps + j*ps]          (panel/StaticPanelMatrix.hpp:178-184)
  * with ld >= rows (col), >= cols (row), >= ps*cols (panel; BLAST calls it the panel "spacing").
  *
- * All floating-point work is IEEE binary64. Results agree with BLAST's algorithm run on the same
- * inputs to a normwise relative error <= 10*n*eps (most kernels reproduce BLAST's order of fused
- * multiply-adds exactly; divisions by a pivot are done as multiplications by its reciprocal).
+ * Results agree with BLAST's algorithm run on the same inputs to a normwise relative error <=
+ * 10*n*eps. Most kernels reproduce BLAST's order of IEEE binary64 fused multiply-adds exactly; Cholesky
+ * divides by a pivot as a multiplication by its reciprocal, and from n = 17 on factors square matrices in
+ * 64-bit fixed point scaled row by row (entries held to 2^-60 of their row's norm), save large uniform
+ * batches of sizes that one binary64 thread per matrix does sooner.
  */
 #ifndef BLASTGPU_H
 #define BLASTGPU_H
@@ -101,9 +103,9 @@ int blastgpu_probe_mma_tflops(int kind, double* tflops, blastgpu_stream_t stream
 /* blastgpu_dposv_strided for operands outside device memory: A and B are read in place and L and
  * X written in place, each element once, from/to any memory the GPU can address (pinned host
  * buffers; on hardware-coherent systems such as GB300 any host allocation), so a host-resident batch
- * is solved in one launch without staging copies. The factorisation re-reads its partial results
- * from the device workspaces L_work (n*n doubles per instance) and X_work (n*nrhs per instance),
- * which must be device memory. Same results as blastgpu_dposv_strided, bit for bit.
+ * is solved without staging copies. Up to n = 64 the working copies are shared memory as a rule;
+ * otherwise the factorisation re-reads its partial results from the device workspaces L_work (n*n
+ * doubles per instance) and X_work (n*nrhs per instance), which must be device memory. Same results as blastgpu_dposv_strided, bit for bit.
  * No reference counterpart (BLAST's matrices are host memory by construction). */
 int blastgpu_dposv_mirror_strided(int n, int nrhs, const double* A, int lda, int64_t stride_a,
                                   const double* B, int ldb, int64_t stride_b, double* L, int ldl,
@@ -113,9 +115,8 @@ int blastgpu_dposv_mirror_strided(int n, int nrhs, const double* A, int lda, int
 /* D = chol(beta*C + alpha*op(A)*op(A)^T), lower triangle; op(A) = A (n x k) or, with trans_a = 1,
  * the transpose of a k x n A. The Riccati-recursion kernel that BLAST benchmarks as syrk followed
  * by potrf (bench/blas/SyrkPotrf.cpp:15-40; BLASFEO's dsyrk_dpotrf_ln,
- * include/blasfeo/blasfeo_api/SyrkPotrf.hpp:15-40), fused: the values of syrkLower
- * (dense/Syrk.hpp:15-145) are formed in the factorisation's register tiles, so the result equals
- * blastgpu_dsyrk_lower_strided then blastgpu_dpotrf_strided bit for bit without storing the sum.
+ * include/blasfeo/blasfeo_api/SyrkPotrf.hpp:15-40): syrkLower (dense/Syrk.hpp:15-145) into D, then
+ * potrf in place; the result equals blastgpu_dsyrk_lower_strided then blastgpu_dpotrf_strided bit for bit.
  * Reads only the lower triangle of C; D may alias C, not A. info[b] as blastgpu_dpotrf_strided. */
 int blastgpu_dsyrk_potrf_strided(int n, int k, int trans_a, double alpha, const double* A, int lda,
                                  int64_t stride_a, double beta, const double* C, int ldc, int64_t stride_c,
