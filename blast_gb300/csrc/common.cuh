@@ -73,7 +73,7 @@ int launch_potrf_fix(const blastgpu_posv_desc* desc, int min_n, int max_n, int32
 int launch_potrf_fix(const blastgpu_posv_bwd_desc* desc, int min_n, int max_n, int32_t* info, int64_t batch,
                      cudaStream_t s);
 
-// Factorisation and, with nrhs > 0, solve in fixed point, two matrices per warp (posv_pair.cu), n <= 64. host: the
+// Factorisation in fixed point and, with nrhs > 0, solve, two matrices per warp (posv_pair.cu), n <= 64. host: the
 // operands are in host memory, which changes the order of loads and stores and no result. L may
 // equal A, X may equal B.
 constexpr int kPairMaxN = 64;

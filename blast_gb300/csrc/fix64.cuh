@@ -13,9 +13,11 @@
 //
 //  * A factor entry is q = l * 2^61 held as q = h * 2^30 + l, two signed 32-bit limbs with
 //    |h| <= 2^30 and |l| <= 2^29: 60 bits relative to the row's norm, where binary64 has 53.
-//  * A dot product keeps sum(h h) in units of 2^-62 and sum(h l + l h) in units of 2^-92, both in 64
-//    bits. |sum(h h)| <= 2^60 for any length; the cross sum is at most 2^60 sqrt(length), so it is
-//    folded into the other one every 32 terms. The l l products (below 2^-64 each) are left out.
+//  * A dot product of two rows keeps sum(h h) in units of 2^-62 and sum(h l + l h) in units of 2^-92, both
+//    in 64 bits. Both rows' norms are below 1/2, so |sum(h h)| <= 2^60 for any length; the cross sum is at
+//    most 2^60 sqrt(length), so it is folded into the other one every 32 terms. The l l products (below
+//    2^-64 each) are left out. Columns of a factor and right-hand sides have no such norm: the
+//    substitutions are not done in this arithmetic.
 //  * A term of the matrix or a remainder is an int64 in units of 2^-62.
 //
 // Errors: an entry is rounded to 2^-61 and a dot product of k terms adds about sqrt(k) * 2^-62, where
@@ -168,18 +170,6 @@ FIX64_FN double entry_to_double(int64_t q, int e) {
 #endif
 }
 
-// q * 2^e, rounded once unless the result is subnormal.
-FIX64_FN double to_double(int64_t q, int e) {
-#ifdef __CUDA_ARCH__
-    double const d = (double)q;
-    int const hi = __double2hiint(d), ex = ((hi >> 20) & 0x7ff) + e;
-    if (ex > 0 && ex < 0x7ff) return d == 0.0 ? 0.0 : __hiloint2double(hi + (e << 20), __double2loint(d));
-    return scalbn(d, e);
-#else
-    return __builtin_ldexp((double)q, e);
-#endif
-}
-
 // A pivot's reciprocal square root 1/sqrt(s * 2^-62) = r * 2^u, r in (1, 2], as two 31-bit limbs of
 // r * 2^61. top = 2^(29 - u).
 struct alignas(16) Rsqrt {
@@ -216,8 +206,7 @@ FIX64_FN Rsqrt pivot_rsqrt(int64_t s) {
 }
 
 // t / sqrt(pivot): a remainder in units of 2^-62 becomes an entry in units of 2^-61, truncated. False if the
-// entry reaches 2^BITS (BITS <= 60).
-template <int BITS>
+// entry reaches 2^kEntryBits.
 FIX64_FN bool scale_entry(int64_t t, Rsqrt y, int64_t& q) {
     bool const ok = (uint32_t)(hi32(t) + y.top) < 2u * (uint32_t)y.top;  // |t| <= 2^(61 - u)
     uint64_t const w = (uint64_t)t << (y.u & 31);
@@ -227,7 +216,7 @@ FIX64_FN bool scale_entry(int64_t t, Rsqrt y, int64_t& q) {
     mad(cross, l, y.h);
     q = cross >> 31;
     mad(q, h, y.h);
-    constexpr uint32_t kMost = uint32_t(1) << (BITS - 32);
+    constexpr uint32_t kMost = uint32_t(1) << (kEntryBits - 32);
     return ok && (uint32_t)hi32(q) + kMost < 2 * kMost;
 }
 

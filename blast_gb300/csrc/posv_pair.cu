@@ -1,18 +1,17 @@
-// Batched binary64 Cholesky factorisation and solve in 64-bit fixed point (fix64.cuh), n <= 64, sm_103a:
+// Batched binary64 Cholesky factorisation in 64-bit fixed point (fix64.cuh) and solve, n <= 64, sm_103a:
 // two matrices per warp, each in shared memory.
 //
 // Reference: blast::potrf (dense/Potrf.hpp:66-106), left-looking, and blast::trsm (dense/Trsm.hpp:17-66)
 // for the solves.
 //
 // What bounds it: integer instructions, 28,000 for two matrices of n = 48 without right-hand sides, a
-// quarter of them the products of block columns, and the chain of pivots, with 8 warps per SM. 50,000
-// matrices of n = 48 with 8 right-hand sides take 3.11 ms (1.24 ms the factor alone) against 4.15 ms for
-// a binary64 thread per matrix, which the binary64 pipe holds at 3.0 ms at best; 10,000 take a half, one
-// matrix of n = 24 21 us a call instead of 53. A matrix has 16 lanes, so that the work on the diagonal,
-// which has 16 rows to share it, fills the warp with two matrices, and a batch of small matrices needs few
-// warps. The matrix is read from memory
-// once and written once; the earlier columns, which a thread per matrix reads again for every strip,
-// stay in shared memory.
+// quarter of them the products of block columns, and the chain of pivots, with 8 warps per SM; then the
+// solves' multiply-adds on the binary64 pipe. 50,000 matrices of n = 48 with 8 right-hand sides take 3.70 ms
+// (1.21 ms the factor alone, 1.78 with one right-hand side) against 4.15 ms for a binary64 thread per matrix;
+// 10,000 take a half, one matrix of n = 24 21 us a call instead of 53. A matrix has 16 lanes, so that the
+// work on the diagonal, which has 16 rows to share it, fills the warp with two matrices, and a batch of
+// small matrices needs few warps. The matrix is read from memory once and written once; the earlier
+// columns, which a thread per matrix reads again for every strip, stay in shared memory.
 //
 // The matrix is cut into 16 x 16 blocks (n rounded up), of which the lower ones are stored, each as 16
 // columns of 17 entries of 8 bytes: the matrix's binary64 entry at first, then the remainder, then the
@@ -24,10 +23,9 @@
 // Each integer sum is exact until it is rounded at the end of these steps, and potrf_fix.cu takes the
 // same steps, so the factor is the same bits from both.
 //
-// Solves, 8 right-hand sides at a time: a right-hand side is a row that follows the same steps (y is
-// the row b^T L^-T), with an exponent of its own for each block of 16 entries, since nothing bounds a
-// solution as the diagonal bounds the factor. A block's entries are first scaled to leave 3 bits for
-// growth; should the triangle of the block need more, the block is solved again with 3 bits more.
+// Solves in binary64, up to 8 right-hand sides at a time, from the factor's blocks converted in place: a
+// solution's entries may lie any number of binades apart, and a column of the factor has no norm that
+// bounds the sums. The binary64 pipe stands idle otherwise.
 #include "common.cuh"
 #include "fix64.cuh"
 
@@ -40,26 +38,33 @@ using fix64::Rsqrt;
 constexpr int kB = 16;      // block size
 constexpr int kMaxN = 64;
 constexpr int kGroup = 8;   // right-hand sides solved together
-constexpr int kFwdBits = 60, kBwdBits = 57;  // rows of L have norm < 1/2, its columns only entries < 1/2
 
-// Shared memory of one matrix with N block columns, in bytes from its start.
+// Shared memory of one matrix with N block columns, in bytes from its start: 13.5 KB at N = 3, so that eight
+// warps fit an SM, two to a scheduler. The reciprocals that the solves need take the place of what follows the
+// blocks, and the right-hand sides that of the diagonal blocks' upper triangles (RhsBlock).
 struct Layout {
-    int rsqrt, scale, bad, rhs, expo, bytes;
+    int rsqrt, scale, bad, bytes;
 };
 constexpr int kS = kB + 1;         // column stride of a block
 constexpr int kBlock = kB * kS;    // entries of a block
 // First entry of block (I, J), J <= I.
 __host__ __device__ __forceinline__ int block_at(int I, int J) { return (I * (I + 1) / 2 + J) * kBlock; }
-__host__ __device__ __forceinline__ Layout layout_of(int N, bool solve) {
+__host__ __device__ __forceinline__ Layout layout_of(int N) {
     Layout l;
     l.rsqrt = 8 * block_at(N, 0);
-    l.scale = l.rsqrt + 16 * kB * N;
+    l.scale = l.rsqrt + 16 * kB;
     l.bad = l.scale + 4 * kB * N;
-    l.rhs = l.bad + kB * N;
-    l.expo = l.rhs + (solve ? 8 * kB * kGroup * N : 0);
-    l.bytes = (l.expo + (solve ? 4 * kGroup * (N + 1) : 0) + 15) & ~15;
+    l.bytes = l.rsqrt + max(8 * kB * N, l.bad + kB * N - l.rsqrt);
     return l;
 }
+
+// Entry i of right-hand side c (< kGroup) of a block, counted from the first entry of the diagonal block: column 8 + c
+// has room for 8 + c entries above its diagonal and one below its last row, column 7 - c for the others.
+struct RhsBlock {
+    int a, b, split;
+    __device__ __forceinline__ explicit RhsBlock(int c) : a((8 + c) * kS), b((7 - c) * kS - 8 - c), split(8 + c) {}
+    __device__ __forceinline__ int operator()(int i) const { return i == kB - 1 ? a + kB : (i < split ? a : b) + i; }
+};
 
 struct PairItem {
     int n, nrhs;
@@ -171,7 +176,7 @@ __device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int col
     for (int j = 0; j < kB; ++j) {
         if (j < cols) {
             int64_t q;
-            bool const ok = fix64::scale_entry<fix64::kEntryBits>(t, y, q);
+            bool const ok = fix64::scale_entry(t, y, q);
             off |= !ok && l16 > j;
             Limbs const v = fix64::split(q);
             blk[j * kS] = fix64::pack(v);
@@ -205,195 +210,124 @@ __device__ __forceinline__ bool solve_block_row(int64_t* row, bool mine, const i
             fix64::mad(c1, x[q].l, d.h);
         }
         int64_t v;
-        ok &= fix64::scale_entry<fix64::kEntryBits>((mine ? row[j * kS] : 0) - fix64::total(hh, c0 + c1), rsq[j], v);
+        ok &= fix64::scale_entry((mine ? row[j * kS] : 0) - fix64::total(hh, c0 + c1), rsq[j], v);
         x[j] = fix64::split(v);
         row[j * kS] = fix64::pack(x[j]);
     }
     return ok;
 }
 
-// Right-hand sides r = rt + 4 i of block J: the remainders at Y (columns of the block, kGroup right-hand
-// sides each) take minus the products with the blocks solved so far, forward L(J, K) y_K for K < J,
-// backward L(I, J)^T x_I for I > J. expo[K][r]: the solved blocks' exponents, expo[N][r] that of block J.
-template <int RA, bool BACK>
-__device__ __forceinline__ void rhs_remainder(const int64_t* P, int64_t* Y, const int* expo, int N, int blocks, int J, int rt,
-                                              int ct) {
-    int64_t acc[RA][4];
-    int ez[RA];
-#pragma unroll
-    for (int i = 0; i < RA; ++i) {
-        ez[i] = expo[N * kGroup + rt + 4 * i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0;
-    }
-    for (int K = BACK ? J + 1 : 0; K < (BACK ? blocks : J); ++K) {
-        int64_t const* cols = BACK ? P + block_at(K, J) + 4 * ct * kS : P + block_at(J, K) + 4 * ct;
-        int64_t const* rows = Y + K * kB * kGroup + rt;
-        int64_t hh[RA][4], cr[RA][4];
-#pragma unroll
-        for (int i = 0; i < RA; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                hh[i][j] = 0;
-                cr[i][j] = fix64::kCrossStart;
-            }
-#pragma unroll 4
-        for (int k = 0; k < kB; ++k) {
-            Limbs v[RA], w[4];
-#pragma unroll
-            for (int i = 0; i < RA; ++i) v[i] = fix64::unpack(rows[4 * i]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = fix64::unpack(cols[BACK ? j * kS : j]);
-            product_step<RA>(hh, cr, v, w);
-            rows += kGroup;
-            cols += BACK ? 1 : kS;
-        }
-#pragma unroll
-        for (int i = 0; i < RA; ++i) {
-            int const d = min(63, ez[i] - expo[K * kGroup + rt + 4 * i]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += fix64::total(hh[i][j], cr[i][j]) >> d;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < RA; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) (Y[(J * kB + 4 * ct + j) * kGroup + rt + 4 * i]) -= acc[i][j];
+// 1 / d, the same bits for d times a power of two.
+__device__ __forceinline__ double pivot_reciprocal(double d) {
+    int const hi = __double2hiint(d), field = (hi >> 20) & 0x7ff;
+    if (hi < 0x00100000 || field == 0x7ff) return 1.0 / d;  // no normal positive number
+    return scalbn(rcp_nr(__hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(d))), 1023 - field);
 }
 
-// One right-hand side of block J (its remainders at y, units of 2^(ez - 62)) against the diagonal block:
-// the solution's limbs in place. Returns its exponent.
-template <bool BACK>
-__device__ __forceinline__ int solve_rhs_block(const int64_t* D, const Rsqrt* rsq, int64_t* y, int ez, int cols) {
-    constexpr int kBits = BACK ? kBwdBits : kFwdBits;
-    int64_t top = 0;
+// X(:, g0 .. g0 + nr - 1) of one matrix (16 lanes; the other matrix of the warp runs the same steps). P: the factor
+// in binary64, zeros from row n on; rd: the reciprocals of its diagonal. RL lanes side by side take a right-hand
+// side each, the others rows of a block of 16, up to 8 sums a lane, kRows rows at a time against the diagonal block. With
+// 8 right-hand sides only the triangles of 4 rows leave lanes idle. Whatever RL, every entry's sum takes the other
+// rows in the order in which they are solved, so a matrix's solution does not depend on its neighbour's.
+template <int RL>
+__device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, int blocks, int n, double* P,
+                                            const double* rd, int l16) {
+    constexpr int kRows = RL >= 4 ? 4 : kB / RL;  // rows solved together
+    constexpr int RW = kRows * RL / kB;           // of which a lane has this many
+    constexpr int kSub = kB / kRows;
+    int const r = l16 % RL, first = l16 / RL * RW;
+    RhsBlock const y(r);
 #pragma unroll
-    for (int j = 0; j < kB; ++j) {
-        int64_t const z = y[j * kGroup];
-        top |= z < 0 ? -z : z;
-    }
-    int shift = (64 - fix64::clz64((uint64_t)top)) - (kBits - 3);
-    for (;;) {
-        asm volatile("" ::: "memory");  // the triangle is read again by a second attempt, not kept in registers
-        Limbs x[kB];
-        bool ok = true;
+    for (int c = 0; c < RL; ++c)
+        for (int J = 0; J < blocks; ++J) {
+            int const i = kB * J + l16;
+            P[block_at(J, J) + RhsBlock(c)(l16)] = c < nr && i < n ? it.B[i + (int64_t)(g0 + c) * it.ldb] : 0.0;
+        }
+    __syncwarp();
+    for (int I = 0; I < blocks; ++I) {
+        double* const D = P + block_at(I, I);
+        double acc[kSub][RW];
 #pragma unroll
-        for (int k = 0; k < kB; ++k) {
-            int const j = BACK ? kB - 1 - k : k;
-            x[j] = Limbs{0, 0};
-            if (j >= cols) continue;  // uniform in the warp
-            int64_t hh = 0, c0 = fix64::kCrossStart, c1 = 0;
+        for (int s = 0; s < kSub; ++s)
 #pragma unroll
-            for (int m = 0; m < k; ++m) {
-                int const q = BACK ? kB - 1 - m : m;
-                Limbs const d = fix64::unpack(BACK ? D[j * kS + q] : D[q * kS + j]);
-                fix64::mad(hh, x[q].h, d.h);
-                fix64::mad(c0, x[q].h, d.l);
-                fix64::mad(c1, x[q].l, d.h);
+            for (int w = 0; w < RW; ++w) acc[s][w] = D[y(kRows * s + first + w)];
+        for (int K = 0; K < I; ++K) {
+            double const* l = P + block_at(I, K) + first;
+            double const* yk = P + block_at(K, K);
+#pragma unroll 8
+            for (int k = 0; k < kB; ++k) {
+                double const v = yk[y(k)];
+#pragma unroll
+                for (int s = 0; s < kSub; ++s)
+#pragma unroll
+                    for (int w = 0; w < RW; ++w) acc[s][w] = fma(-l[k * kS + kRows * s + w], v, acc[s][w]);
             }
-            int64_t const z = y[j * kGroup], zs = shift > 0 ? z >> min(shift, 63) : z << -shift;
-            int64_t v;
-            ok &= fix64::scale_entry<kBits>(zs - fix64::total(hh, c0 + c1), rsq[j], v);
-            x[j] = fix64::split(v);
         }
-        if (ok || shift > 200) {
 #pragma unroll
-            for (int j = 0; j < kB; ++j) y[j * kGroup] = fix64::pack(x[j]);
-            return ez + shift;
-        }
-        shift += 3;
-    }
-}
-
-// X(:, g0 .. g0 + nr - 1) of one matrix (16 lanes; the other matrix of the warp runs the same steps).
-template <int RA>
-__device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, int N, int blocks, int nmax, int n, bool good, const int64_t* P,
-                                            const Rsqrt* rsq, const int* scale, int64_t* Y, int* expo, int l16) {
-    int const rt = l16 & 3, ct = l16 >> 2;
-    bool const mine = l16 < nr;  // this lane's right-hand side
-    int const r = l16 & (kGroup - 1);
-    int top = -100000;  // largest exponent of the solved blocks
-    bool finite = true;
-    for (int J = 0; J < blocks; ++J) {
-        int64_t* y = Y + J * kB * kGroup;
-        int const cols = min(kB, nmax - kB * J);
-        int ez = 0;
-        if (l16 < kGroup) {
-            double b[kB];
-            int eb = -100000;
+        for (int j = 0; j < kB; ++j) {
+            int const sj = j / kRows, jj = j % kRows;
+            double const v = __shfl_sync(0xffffffffu, acc[sj][jj % RW] * rd[kB * I + j], jj / RW * RL + r, kB);
 #pragma unroll
-            for (int j = 0; j < kB; ++j) {
-                int const i = kB * J + j;
-                b[j] = mine && i < n ? it.B[i + (int64_t)(g0 + r) * it.ldb] : 0.0;
-            }
+            for (int s = sj; s < kSub; ++s)
 #pragma unroll
-            for (int j = 0; j < kB; ++j) {
-                int const field = (__double2hiint(b[j]) >> 20) & 0x7ff;
-                finite &= field != 0x7ff;
-                int const e = b[j] == 0.0 ? -100000 : max(field, 1) - 1022 - scale[kB * J + j];
-                eb = max(eb, e);
-            }
-            ez = max(eb, top) + 2;
+                for (int w = 0; w < RW; ++w) {
+                    if (s == sj && first + w == jj) acc[s][w] = v;
+                    else if (s > sj || first + w > jj) acc[s][w] = fma(-D[j * kS + kRows * s + first + w], v, acc[s][w]);
+                }
+        }
 #pragma unroll
-            for (int j = 0; j < kB; ++j) {
-                int64_t v;
-                fix64::from_double(b[j], scale[kB * J + j] + ez, v);
-                (y[j * kGroup + r]) = v;
-            }
-            expo[N * kGroup + r] = ez;
-        }
-        __syncwarp();
-        if (J > 0) {
-            rhs_remainder<RA, false>(P, Y, expo, N, blocks, J, rt, ct);
-            __syncwarp();
-        }
-        if (l16 < kGroup) {
-            int const e = solve_rhs_block<false>(P + block_at(J, J), rsq + kB * J, y + r, ez, cols);
-            expo[J * kGroup + r] = e;
-            top = max(top, e);
-        }
+        for (int s = 0; s < kSub; ++s)
+#pragma unroll
+            for (int w = 0; w < RW; ++w)
+                if (kB * I + kRows * s + first + w < n) D[y(kRows * s + first + w)] = acc[s][w];
         __syncwarp();
     }
-    top = -100000;
-    for (int J = blocks - 1; J >= 0; --J) {
-        int64_t* y = Y + J * kB * kGroup;
-        int const cols = min(kB, nmax - kB * J);
-        int ez = 0;
-        if (l16 < kGroup) {
-            int const ey = expo[J * kGroup + r];
-            ez = max(ey, top) + 2;
-            int const d = min(63, ez - ey - 1);
+    for (int I = blocks - 1; I >= 0; --I) {
+        double* const D = P + block_at(I, I);
+        double acc[kSub][RW];
 #pragma unroll
-            for (int j = 0; j < kB; ++j) (y[j * kGroup + r]) = fix64::join(fix64::unpack(y[j * kGroup + r])) >> d;
-            expo[N * kGroup + r] = ez;
+        for (int s = 0; s < kSub; ++s)
+#pragma unroll
+            for (int w = 0; w < RW; ++w) acc[s][w] = D[y(kRows * s + first + w)];
+        for (int K = blocks - 1; K > I; --K) {
+            double const* l = P + block_at(K, I) + first * kS;
+            double const* yk = P + block_at(K, K);
+#pragma unroll 8
+            for (int k = kB - 1; k >= 0; --k) {
+                double const v = yk[y(k)];
+#pragma unroll
+                for (int s = 0; s < kSub; ++s)
+#pragma unroll
+                    for (int w = 0; w < RW; ++w) acc[s][w] = fma(-l[(kRows * s + w) * kS + k], v, acc[s][w]);
+            }
         }
-        __syncwarp();
-        if (J + 1 < blocks) {
-            rhs_remainder<RA, true>(P, Y, expo, N, blocks, J, rt, ct);
-            __syncwarp();
+#pragma unroll
+        for (int j = kB - 1; j >= 0; --j) {
+            int const sj = j / kRows, jj = j % kRows;
+            double const v = __shfl_sync(0xffffffffu, acc[sj][jj % RW] * rd[kB * I + j], jj / RW * RL + r, kB);
+#pragma unroll
+            for (int s = sj; s >= 0; --s)
+#pragma unroll
+                for (int w = 0; w < RW; ++w) {
+                    if (s == sj && first + w == jj) acc[s][w] = v;
+                    else if (s < sj || first + w < jj) acc[s][w] = fma(-D[(kRows * s + first + w) * kS + j], v, acc[s][w]);
+                }
         }
-        if (l16 < kGroup) {
-            int const e = solve_rhs_block<true>(P + block_at(J, J), rsq + kB * J, y + r, ez, cols);
-            expo[J * kGroup + r] = e;
-            top = max(top, e);
-        }
+#pragma unroll
+        for (int s = 0; s < kSub; ++s)
+#pragma unroll
+            for (int w = 0; w < RW; ++w)
+                if (kB * I + kRows * s + first + w < n) D[y(kRows * s + first + w)] = acc[s][w];
         __syncwarp();
     }
     // X in whole lines, 16 lanes along a column (one lane per right-hand side writes 8 bytes to a line: 0.9 ms
     // more for 10,000 matrices with X in host memory).
 #pragma unroll
-    for (int c = 0; c < kGroup; ++c) {
-        bool const ok = __shfl_sync(0xffffffffu, finite, c, kB) && good;
-        if (c < nr) {
-            for (int J = 0; J < blocks; ++J) {
-                int const i = kB * J + l16;
-                if (i < n) {
-                    double const x = fix64::to_double(fix64::join(fix64::unpack(Y[i * kGroup + c])), expo[J * kGroup + c] - 61 - scale[i]);
-                    it.X[i + (int64_t)(g0 + c) * it.ldx] = ok ? x : __longlong_as_double(0x7ff8000000000000ll);
-                }
-            }
+    for (int c = 0; c < RL; ++c)
+        for (int J = 0; J < blocks; ++J) {
+            int const i = kB * J + l16;
+            if (c < nr && i < n) it.X[i + (int64_t)(g0 + c) * it.ldx] = P[block_at(J, J) + RhsBlock(c)(l16)];
         }
-    }
     __syncwarp();
 }
 
@@ -422,14 +356,12 @@ template <bool SOLVE, bool HOST, class Batch>
 __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t count, int N, int32_t* info) {
     extern __shared__ __align__(16) unsigned char smem[];
     int const l16 = threadIdx.x & 15, half = threadIdx.x >> 4;
-    Layout const lay = layout_of(N, SOLVE);
+    Layout const lay = layout_of(N);
     unsigned char* base = smem + half * lay.bytes;
     int64_t* P = reinterpret_cast<int64_t*>(base);
     Rsqrt* rsq = reinterpret_cast<Rsqrt*>(base + lay.rsqrt);
     int* scale = reinterpret_cast<int*>(base + lay.scale);
     unsigned char* bad = base + lay.bad;
-    int64_t* Y = reinterpret_cast<int64_t*>(base + lay.rhs);
-    int* expo = reinterpret_cast<int*>(base + lay.expo);
     int64_t const b = 2 * (int64_t)blockIdx.x + half;
     PairItem it;
     it.n = 0, it.nrhs = 0;
@@ -499,10 +431,10 @@ __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t 
             else block_remainder<4>(P, n, I, J, scale, bad, l16 & 3, l16 >> 2);
         }
         __syncwarp();
-        factor_diagonal(P + block_at(J, J), kB * J, min(kB, nmax - kB * J), rsq + kB * J, bad + kB * J, l16, fail);
+        factor_diagonal(P + block_at(J, J), kB * J, min(kB, nmax - kB * J), rsq, bad + kB * J, l16, fail);
         __syncwarp();
         for (int I = J + 1; I < blocks; ++I)
-            if (!solve_block_row(P + block_at(I, J) + l16, kB * I + l16 < nmax, P + block_at(J, J), rsq + kB * J)) bad[kB * I + l16] = fix64::kNoPivot | fix64::kOutOfRange;
+            if (!solve_block_row(P + block_at(I, J) + l16, kB * I + l16 < nmax, P + block_at(J, J), rsq)) bad[kB * I + l16] = fix64::kNoPivot | fix64::kOutOfRange;
         __syncwarp();
         if constexpr (HOST) store_columns(it, n, J, blocks, fail, P, scale, bad, l16);
     }
@@ -513,31 +445,35 @@ __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t 
     if constexpr (HOST)
         for (int i = l16; i < n; i += kB) again |= (bad[i] & fix64::kOutOfRange) != 0;
     again = __any_sync(0xffffffffu, again);
-    for (int I = 0; I < (again ? blocks : 0); ++I) {
+    for (int I = 0; I < (again || SOLVE ? blocks : 0); ++I) {
         int const r = kB * I + l16, e = scale[r] - 61, first_nan = (bad[r] & fix64::kOutOfRange) ? 0 : fail;
-        if (r < n) {
-            for (int J = 0; J <= I; ++J) {
-                int64_t const* blk = P + block_at(I, J) + l16;
-                double* l = it.L + r + (int64_t)(kB * J) * it.ldl;
+        for (int J = 0; J <= I; ++J) {
+            int64_t* blk = P + block_at(I, J) + l16;
+            double* l = it.L + r + (int64_t)(kB * J) * it.ldl;
 #pragma unroll 4
-                for (int c = 0; c < kB; ++c) {
-                    int const col = kB * J + c;
-                    double const x = fix64::entry_to_double(fix64::join(fix64::unpack(blk[c * kS])), e);
-                    if (col <= r) l[c * it.ldl] = col >= first_nan ? __longlong_as_double(0x7ff8000000000000ll) : x;
-                }
+            for (int c = 0; c < kB; ++c) {
+                int const col = kB * J + c;
+                double x = fix64::entry_to_double(fix64::join(fix64::unpack(blk[c * kS])), e);
+                if (col >= first_nan) x = __longlong_as_double(0x7ff8000000000000ll);
+                if (SOLVE && col <= r) blk[c * kS] = r < n ? __double_as_longlong(x) : 0;
+                if (again && col <= r && r < n) l[c * it.ldl] = x;
             }
         }
     }
     if constexpr (SOLVE) {
-        // rows past n: their remainders are 0, and so are the solutions' entries; the pivots must exist
-        for (int i = n + l16; i < kB * blocks; i += kB) rsq[i] = Rsqrt{0, int32_t(1) << 30, 0, int32_t(1) << 29};
+        double* F = reinterpret_cast<double*>(P);
+        double* rd = reinterpret_cast<double*>(rsq);
         __syncwarp();
+        for (int i = l16; i < kB * blocks; i += kB)
+            rd[i] = i < n ? pivot_reciprocal(F[block_at(i / kB, i / kB) + i % kB * (kS + 1)]) : 1.0;
         int const nrhs = have ? it.nrhs : 0;
         int const most = max(nrhs, __shfl_xor_sync(0xffffffffu, nrhs, 16));
         for (int g0 = 0; g0 < most; g0 += kGroup) {
-            int const nr = max(0, min(kGroup, nrhs - g0));
-            if (min(kGroup, most - g0) <= 4) solve_group<1>(it, g0, nr, N, blocks, nmax, n, fail == n, P, rsq, scale, Y, expo, l16);
-            else solve_group<2>(it, g0, nr, N, blocks, nmax, n, fail == n, P, rsq, scale, Y, expo, l16);
+            int const nr = max(0, min(kGroup, nrhs - g0)), wide = min(kGroup, most - g0);
+            if (wide > 4) solve_group<8>(it, g0, nr, blocks, n, F, rd, l16);
+            else if (wide > 2) solve_group<4>(it, g0, nr, blocks, n, F, rd, l16);
+            else if (wide == 2) solve_group<2>(it, g0, nr, blocks, n, F, rd, l16);
+            else solve_group<1>(it, g0, nr, blocks, n, F, rd, l16);
         }
     }
 }
@@ -564,13 +500,17 @@ struct PairDesc {
     }
 };
 
+constexpr size_t kFourPerSm = 48 * 1024;
+
 template <bool SOLVE, bool HOST = false, class Batch>
 int launch(Batch const& batch, int max_n, int64_t count, int32_t* info, cudaStream_t s) {
     if (count == 0) return BLASTGPU_SUCCESS;
     if (max_n > kMaxN || (count + 1) / 2 > 0x7fffffff) return BLASTGPU_ERR_TOO_LARGE;
     int const N = (max_n + kB - 1) / kB;
-    size_t const smem = 2 * (size_t)layout_of(N, SOLVE).bytes;
-    cudaError_t const e = ensure_smem<posv_pair_kernel<SOLVE, HOST, Batch>>(2 * (size_t)layout_of(kMaxN / kB, SOLVE).bytes);
+    // At N = 4 a fifth warp fits an SM, which helps the solves (n = 64 x 20,000: 3.0 ms, 3.4 with four) and leaves the
+    // schedulers uneven for the factor alone (n = 60 x 20,000: 1.49 ms, 1.33 with four).
+    size_t const smem = SOLVE || N < 4 ? 2 * (size_t)layout_of(N).bytes : kFourPerSm;
+    cudaError_t const e = ensure_smem<posv_pair_kernel<SOLVE, HOST, Batch>>(kFourPerSm);
     if (e != cudaSuccess) { set_cuda_error(e); return BLASTGPU_ERR_CUDA; }
     posv_pair_kernel<SOLVE, HOST, Batch><<<(unsigned)((count + 1) / 2), 32, smem, s>>>(batch, count, N, info);
     return check_launch();

@@ -341,7 +341,7 @@ __device__ __forceinline__ int factor_diagonal(int k0, int mr, int nb, const int
     for (int j = 0; j < kNB; ++j) {
         if (j < done) {  // warp-uniform
             int64_t q;
-            bool const ok = fix64::scale_entry<fix64::kEntryBits>(t, y, q);
+            bool const ok = fix64::scale_entry(t, y, q);
             off |= !ok && lane > j;
             Limbs const v = fix64::split(q);
             if (lane >= j && mine) W[(k0 + lane) + (int64_t)(k0 + j) * ldw] = S::kTensor ? fix64::to_digits(q) : fix64::pack(v);
@@ -388,7 +388,7 @@ __device__ __forceinline__ void solve_row(int row, int r, int k0, int done, cons
         }
         int64_t const t = C[j * S::CS + r] - fix64::total(hh, c0 + c1);
         int64_t v;
-        bool const in = fix64::scale_entry<fix64::kEntryBits>(t, rsq[j], v);
+        bool const in = fix64::scale_entry(t, rsq[j], v);
         x[j] = fix64::split(v);
         if (j < done) {
             ok &= in;
