@@ -22,6 +22,22 @@
 //
 // Errors: an entry is rounded to 2^-61 and a dot product of k terms adds about sqrt(k) * 2^-62, where
 // binary64 rounds every partial sum to 2^-53 of its size.
+//
+// That is an error of 2^-61 or so of s_i s_j, whatever the sizes of the terms of entry (i, j), while
+// binary64's follows them down. Where unknowns are coupled weakly (a kernel's far points, blocks with a
+// small entry between them), the solution's small entries come from such small terms. So the kernels
+// certify what they factor here, panel by panel, and leave the rest of a matrix to binary64 where
+//  * an entry's terms |l_ik l_jk| are all below a threshold, the last one, |l_ij l_jj|, among them (weak()),
+//    and i and j are not both coupled to another unknown of the panel with |l_ik l_kj| above it either,
+//    through which binary64's errors reach the same unknowns. An entry of zero with no term at all is exact.
+//    The threshold is 2^-16 at n = 17 and falls with n, so that the error is at most about 10 n 2^-52 of the
+//    terms (weak_shift()). Gaussian and Riccati matrices have no such entry in thousands, and one or two
+//    weak entries to look at from n = 48 on;
+//  * a pivot is below 2^-42 of its diagonal entry or so (kPivotMin): whether it is positive is then for
+//    binary64's own rounding to say;
+//  * a row has an entry out of range, or entries whose squares exceed its diagonal entry (kNormMost): the
+//    matrix is not positive definite, and sums might wrap;
+//  * a diagonal entry is zero, negative or not finite.
 #pragma once
 
 #include <stdint.h>
@@ -39,8 +55,9 @@ struct Limbs {
     int32_t l, h;  // q = h * 2^30 + l
 };
 
-// Factor entries of a positive definite matrix stay below 2^60.
-constexpr int kEntryBits = 60;
+// Factor entries of a positive definite matrix stay below 2^60. (2^32 less is asked for, so that a high limb is
+// below 2^30.)
+constexpr int64_t kEntryMost = (int64_t(1) << 60) - (int64_t(1) << 32);
 // Terms after which the cross sum is folded.
 constexpr int kFold = 32;
 
@@ -124,28 +141,40 @@ FIX64_FN void fold(int64_t& hh, int64_t& cross) {
     cross &= (int64_t(1) << 30) - 1;
 }
 
-// floor(log2 |a|) for finite a; far below any other for zero, 0 for infinities and NaN.
-FIX64_FN int exponent_of(double a) {
-    uint64_t const u = bits_of(a) << 1;
-    int const field = (int)(u >> 53);
-    if (field == 0x7ff) return 0;
-    if (u == 0) return -100000;
-    return field != 0 ? field - 1023 : -1011 - clz64(u);
-}
-
 // Scale exponent of a row from its diagonal entry: a_ii * 4^-e in [1/16, 1/4). False for a diagonal
-// that no positive definite matrix has (zero, negative, infinite, NaN); e then brings |a_ii| below 1/4.
+// that no positive definite matrix has (zero, negative, infinite, NaN).
 FIX64_FN bool scale_exponent(double aii, int& e) {
     uint64_t const u = bits_of(aii);
-    e = u << 1 == 0 ? -600 : (exponent_of(aii) + 4) >> 1;
-    return (u >> 52) < 0x7ff && u != 0;
+    int const field = (int)(u >> 52);
+    if (field >= 0x7ff || u == 0) {
+        e = 0;
+        return false;
+    }
+    e = ((field != 0 ? field - 1023 : -1011 - clz64(u)) + 4) >> 1;  // floor(log2 aii) + 4, halved
+    return true;
 }
 
-// What is known of a row: its pivot cannot be positive; its entries left the fixed-point range.
-constexpr unsigned char kNoPivot = 1, kOutOfRange = 2;
-// A row without a usable diagonal takes its scale from its other entries, with room for the growth that
-// nothing bounds any more.
-constexpr int kGrowth = 12;
+// The threshold below which an entry is weak is 2^-(16 + weak_shift(n)): 2^-61 of error is 10 n 2^-52 of it, or less.
+FIX64_FN int weak_shift(int n) { return (n >= 34) + (n >= 68) + (n >= 136) + (n >= 272); }
+// Whether |t| is below it (t, an entry's remainder l_ij l_jj, in units of 2^-62; below: weak_below(n)).
+FIX64_FN uint32_t weak_below(int n) { return (uint32_t(1) << 14) >> weak_shift(n); }
+FIX64_FN bool weak(int64_t t, uint32_t below) { return (uint32_t)hi32(t) + below < 2 * below; }
+// Whether the product of two entries with these high limbs is above it.
+FIX64_FN bool strong(int32_t h1, int32_t h2, uint32_t below) {
+    uint64_t const a = (uint32_t)(h1 < 0 ? -h1 : h1), b = (uint32_t)(h2 < 0 ? -h2 : h2);
+    return (uint32_t)(a * b >> 32) >= below;
+}
+FIX64_FN int32_t high_limb(int64_t q) { return (int32_t)(q >> 30); }
+
+// Sum of squares of the high limbs of a row's entries in a panel: 16 of them fit 64 bits without a sign, and
+// norm_of makes units of 2^-26 of them.
+FIX64_FN void add_square(int64_t& sum, int32_t h) { mad(sum, h, h); }
+FIX64_FN uint32_t norm_of(int64_t sum) { return (uint32_t)((uint64_t)sum >> 36); }
+// 1/4, and more than what rounding the limbs may add.
+constexpr uint32_t kNormMost = (uint32_t(1) << 24) + (uint32_t(1) << 10);
+// A row's word: the sum of squares, whether it has had an entry other than zero, and whether its entries
+// of the panel at hand are left to binary64.
+constexpr uint32_t kNormMask = (uint32_t(1) << 28) - 1, kSeen = uint32_t(1) << 28, kTodo = uint32_t(1) << 29;
 
 // a * 2^-scale in units of 2^-62 (scale = e_i + e_j), truncated. False if |a| * 2^-scale is not below
 // 1/4 (or a is not finite): the matrix is then not positive definite.
@@ -176,8 +205,9 @@ struct alignas(16) Rsqrt {
     int32_t l, h, u, top;
 };
 
-// Remainders below this are no positive pivots: 2^-60 of the diagonal entry's size.
-constexpr int64_t kPivotMin = 4;
+// The smallest pivot, 2^-42 to 2^-40 of its diagonal entry. Binary64's error of a pivot is at most about
+// (n + 1) 2^-53 of the diagonal entry, 2^-44 for n = 512, so above this both find it positive.
+constexpr int64_t kPivotMin = int64_t(1) << 18;
 
 // s in [kPivotMin, 2^62). Halley's iteration (one term beyond Newton) on the hardware's binary32
 // estimate: with e = 1 - v y^2, y (1 + e/2 + 3 e^2/8) has a relative error of 5/16 |e|^3, below
@@ -206,7 +236,7 @@ FIX64_FN Rsqrt pivot_rsqrt(int64_t s) {
 }
 
 // t / sqrt(pivot): a remainder in units of 2^-62 becomes an entry in units of 2^-61, truncated. False if the
-// entry reaches 2^kEntryBits.
+// entry reaches kEntryMost.
 FIX64_FN bool scale_entry(int64_t t, Rsqrt y, int64_t& q) {
     bool const ok = (uint32_t)(hi32(t) + y.top) < 2u * (uint32_t)y.top;  // |t| <= 2^(61 - u)
     uint64_t const w = (uint64_t)t << (y.u & 31);
@@ -216,7 +246,7 @@ FIX64_FN bool scale_entry(int64_t t, Rsqrt y, int64_t& q) {
     mad(cross, l, y.h);
     q = cross >> 31;
     mad(q, h, y.h);
-    constexpr uint32_t kMost = uint32_t(1) << (kEntryBits - 32);
+    constexpr uint32_t kMost = (uint32_t)(kEntryMost >> 32);
     return ok && (uint32_t)hi32(q) + kMost < 2 * kMost;
 }
 

@@ -21,13 +21,15 @@
 //  * the diagonal block: a row per lane, right-looking in registers, the pivot row's limbs by shuffles;
 //  * the blocks below: a row per lane against the diagonal block.
 // Each integer sum is exact until it is rounded at the end of these steps, and potrf_fix.cu takes the
-// same steps, so the factor is the same bits from both.
+// same steps, so the factor is the same bits from both. A matrix whose block column cannot be certified
+// (fix64.cuh) has its columns from there on factored in binary64 (potrf_strips.cuh) at the end, by its 16 lanes.
 //
 // Solves in binary64, up to 8 right-hand sides at a time, from the factor's blocks converted in place: a
 // solution's entries may lie any number of binades apart, and a column of the factor has no norm that
 // bounds the sums. The binary64 pipe stands idle otherwise.
 #include "common.cuh"
 #include "fix64.cuh"
+#include "potrf_strips.cuh"
 
 namespace blastgpu {
 namespace {
@@ -43,7 +45,7 @@ constexpr int kGroup = 8;   // right-hand sides solved together
 // warps fit an SM, two to a scheduler. The reciprocals that the solves need take the place of what follows the
 // blocks, and the right-hand sides that of the diagonal blocks' upper triangles (RhsBlock).
 struct Layout {
-    int rsqrt, scale, bad, bytes;
+    int rsqrt, scale, row, bytes;
 };
 constexpr int kS = kB + 1;         // column stride of a block
 constexpr int kBlock = kB * kS;    // entries of a block
@@ -53,8 +55,8 @@ __host__ __device__ __forceinline__ Layout layout_of(int N) {
     Layout l;
     l.rsqrt = 8 * block_at(N, 0);
     l.scale = l.rsqrt + 16 * kB;
-    l.bad = l.scale + 4 * kB * N;
-    l.bytes = l.rsqrt + max(8 * kB * N, l.bad + kB * N - l.rsqrt);
+    l.row = l.scale + 4 * kB * N;
+    l.bytes = l.rsqrt + max(8 * kB * N, l.row + 4 * kB * N - l.rsqrt);
     return l;
 }
 
@@ -93,20 +95,19 @@ __device__ __forceinline__ void product_step(int64_t (&hh)[RA][4], int64_t (&cr)
 }
 
 // Block (I, J) of the matrix: binary64 entries to the remainders A - L L^T over the block columns
-// before J, for the block's first 4 RA rows.
+// before J, for the block's first 4 RA rows. False if an entry is out of range.
 template <int RA>
-__device__ __forceinline__ void block_remainder(int64_t* P, int n, int I, int J, const int* scale, unsigned char* bad,
-                                                int rt, int ct) {
+__device__ __forceinline__ bool block_remainder(int64_t* P, int n, int I, int J, const int* scale, int rt, int ct) {
     int64_t* blk = P + block_at(I, J) + 4 * ct * kS + rt;
     int64_t hh[RA][4], cr[RA][4];
     int ec[4];
+    bool ok = true;
 #pragma unroll
     for (int j = 0; j < 4; ++j) ec[j] = scale[kB * J + 4 * ct + j];
 #pragma unroll
     for (int i = 0; i < RA; ++i) {
         int const row = kB * I + rt + 4 * i, er = scale[row];
         int const cols = row < n ? row - kB * J - 4 * ct : -1;  // columns 0 .. cols of this lane's four exist
-        bool ok = true;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             int64_t v;
@@ -115,7 +116,6 @@ __device__ __forceinline__ void block_remainder(int64_t* P, int n, int I, int J,
             hh[i][j] = j <= cols ? -v : 0;
             cr[i][j] = fix64::kCrossStart;
         }
-        if (!ok) bad[row] = fix64::kNoPivot | fix64::kOutOfRange;
     }
     for (int K = 0; K < J; ++K) {
         int64_t const* rows = P + block_at(I, K) + rt;
@@ -142,13 +142,20 @@ __device__ __forceinline__ void block_remainder(int64_t* P, int n, int I, int J,
     for (int i = 0; i < RA; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) blk[j * kS + 4 * i] = -fix64::total(hh[i][j], cr[i][j]);
+    return ok;
 }
 
-// A diagonal block, a row per lane (16 lanes per matrix), right-looking. fail: the first column whose pivot
-// is not positive (unchanged if there is none); what follows it is not used. first: the block's first
-// column; cols: columns of the block that some matrix of the warp has.
-__device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int cols, Rsqrt* rsq, unsigned char* bad, int l16,
-                                                int& fail) {
+// A row's sum of squares and whether it has had an entry (fix64.cuh) after a panel; false if the sum is too large.
+__device__ __forceinline__ bool add_row(uint32_t& row, int64_t squares, int any) {
+    row = (row + fix64::norm_of(squares)) | (any != 0 ? fix64::kSeen : 0);
+    return (row & fix64::kNormMask) <= fix64::kNormMost;
+}
+
+// A diagonal block, a row per lane (16 lanes per matrix), right-looking. rows: rows of the block that the matrix
+// has; cols: columns that some matrix of the warp has. False if a pivot is too small, or the lane's row out of
+// range; what follows is not used then. weak: the row's entries that need a look (served).
+__device__ __forceinline__ bool factor_diagonal(int64_t* blk, int rows, int cols, Rsqrt* rsq, uint32_t& row, int l16,
+                                                uint32_t below, unsigned& weak) {
     blk += l16;
     int64_t acc[kB], cr[kB];
 #pragma unroll
@@ -156,20 +163,18 @@ __device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int col
         acc[c] = l16 < cols ? blk[c * kS] : 0;
         cr[c] = -fix64::kCrossStart;
     }
-    bool const no_pivot = bad[l16] != 0;
-    bool off = false;
+    bool good = true, off = false;
+    int64_t squares = 0;
+    int any = 0;
     // The next pivot's reciprocal square root is taken as soon as its column is up to date, beside the
     // products of the columns after it.
     int64_t t = 0;
     Rsqrt y;
     auto pivot = [&](int c) {
         t = acc[c] - fix64::total(0, -cr[c]);
-        int64_t s = __shfl_sync(0xffffffffu, off || no_pivot ? (int64_t)-1 : t, c, kB);
-        if (s < fix64::kPivotMin) {
-            fail = min(fail, first + c);
-            s = int64_t(1) << 60;
-        }
-        y = fix64::pivot_rsqrt(s);
+        int64_t const s = __shfl_sync(0xffffffffu, t, c, kB);
+        good &= s >= fix64::kPivotMin || c >= rows;
+        y = fix64::pivot_rsqrt(max(s, fix64::kPivotMin));
     };
     pivot(0);
 #pragma unroll
@@ -177,9 +182,14 @@ __device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int col
         if (j < cols) {
             int64_t q;
             bool const ok = fix64::scale_entry(t, y, q);
-            off |= !ok && l16 > j;
             Limbs const v = fix64::split(q);
             blk[j * kS] = fix64::pack(v);
+            if (fix64::weak(t, below)) weak |= 1u << j;
+            if (l16 >= j) {
+                off |= !ok;
+                fix64::add_square(squares, v.h);
+                any |= v.h | v.l;
+            }
             if (l16 == 0) rsq[j] = y;
             int const nh = -v.h, nl = -v.l;
 #pragma unroll
@@ -192,13 +202,19 @@ __device__ __forceinline__ void factor_diagonal(int64_t* blk, int first, int col
             }
         }
     }
-    if (off) bad[l16] = fix64::kNoPivot | fix64::kOutOfRange;
+    weak &= l16 < rows ? (1u << l16) - 1 : 0;
+    if (l16 >= rows) return good;
+    return add_row(row, squares, any) && good && !off;
 }
 
-// A row (this lane's, at row) against the diagonal block D; mine: the row exists (else it becomes zeros).
-__device__ __forceinline__ bool solve_block_row(int64_t* row, bool mine, const int64_t* D, const Rsqrt* rsq) {
+// A row (this lane's, at x) against the diagonal block D; mine: the row exists (else it becomes zeros). False if
+// it is out of range.
+__device__ __forceinline__ bool solve_block_row(int64_t* x_at, bool mine, const int64_t* D, const Rsqrt* rsq, uint32_t& row,
+                                                uint32_t below, unsigned& weak) {
     Limbs x[kB];
     bool ok = true;
+    int64_t squares = 0;
+    int any = 0;
 #pragma unroll
     for (int j = 0; j < kB; ++j) {
         int64_t hh = 0, c0 = fix64::kCrossStart, c1 = 0;
@@ -210,11 +226,49 @@ __device__ __forceinline__ bool solve_block_row(int64_t* row, bool mine, const i
             fix64::mad(c1, x[q].l, d.h);
         }
         int64_t v;
-        ok &= fix64::scale_entry((mine ? row[j * kS] : 0) - fix64::total(hh, c0 + c1), rsq[j], v);
+        int64_t const t = (mine ? x_at[j * kS] : 0) - fix64::total(hh, c0 + c1);
+        ok &= fix64::scale_entry(t, rsq[j], v);
+        if (fix64::weak(t, below)) weak |= 1u << j;
         x[j] = fix64::split(v);
-        row[j * kS] = fix64::pack(x[j]);
+        x_at[j * kS] = fix64::pack(x[j]);
+        fix64::add_square(squares, x[j].h);
+        any |= x[j].h | x[j].l;
     }
-    return ok;
+    return add_row(row, squares, any) && ok;
+}
+
+// Whether the weak entries of rows first + l16 (a lane's, those of n) in block column J are served by fixed point all
+// the same (fix64.cuh). row: the rows' words; A: the matrix. A row without any entry so far is its lane's affair; other
+// entries are looked at by their matrix's 16 lanes together, one entry of each matrix at a time.
+__device__ __forceinline__ bool served(const int64_t* P, const uint32_t* row, const double* A, int64_t lda, int n, int first,
+                                       int J, uint32_t below, unsigned weak, int l16) {
+    int const base = kB * J, shift = threadIdx.x & 16;
+    auto entry = [&](int r, int c) { return P[block_at(r / kB, c / kB) + c % kB * kS + r % kB]; };
+    auto half = [&](bool x) { return (__ballot_sync(0xffffffffu, x) >> shift) & 0xffffu; };
+    bool ok = true;
+    if (weak != 0 && (row[first + l16] & fix64::kSeen) == 0) {
+        for (; weak != 0; weak &= weak - 1) ok &= A[first + l16 + (base + __ffs(weak) - 1) * lda] == 0.0;
+    }
+    for (;;) {
+        unsigned const who = half(weak != 0);
+        if (!__any_sync(0xffffffffu, who != 0)) return ok;
+        int const src = max(__ffs(who) - 1, 0), i = first + src;
+        int const j = base + max(__ffs(__shfl_sync(0xffffffffu, weak, src, kB)) - 1, 0);
+        unsigned through = 0, terms = 0;
+        auto look = [&](int k) {
+            int64_t a = 0, b = 0;
+            if (who != 0 && k < n && k != i && k != j) a = entry(max(i, k), min(i, k)), b = entry(max(j, k), min(j, k));
+            through |= half(fix64::strong(fix64::unpack(a).h, fix64::unpack(b).h, below));
+            terms |= half(k < j && a != 0 && b != 0);
+        };
+        look(base + l16);
+        if (__any_sync(0xffffffffu, who != 0 && through == 0)) {
+            for (int K = 0; K < J; ++K) look(kB * K + l16);
+            // an entry of zero without terms is exact
+            if (l16 == src && who != 0 && through == 0 && (terms != 0 || entry(i, j) != 0 || A[i + j * lda] != 0.0)) ok = false;
+        }
+        if (l16 == src) weak = ok ? weak & (weak - 1) : 0;
+    }
 }
 
 // 1 / d, the same bits for d times a power of two.
@@ -337,23 +391,19 @@ __device__ __forceinline__ void solve_group(PairItem const& it, int g0, int nr, 
 // right-hand sides take 4.91 ms with three batches in flight and 5.11 alone (row blocks of A read, and L written,
 // at once: 5.25, 5.50), 10,000 1.18 ms (1.29), 30,000 of n = 60 5.2 (5.6); prefetches into L2 gave nothing.
 // Columns kB J .. kB J + 15 of the factor:
-__device__ __forceinline__ void store_columns(PairItem const& it, int n, int J, int blocks, int fail, const int64_t* P,
-                                              const int* scale, const unsigned char* bad, int l16) {
+__device__ __forceinline__ void store_columns(PairItem const& it, int n, int J, const int64_t* P, const int* scale, int l16) {
     for (int col = kB * J; col < min(n, kB * J + kB); ++col) {
         double* l = it.L + (int64_t)col * it.ldl;
         int const at = (int)(reinterpret_cast<uintptr_t>(l) >> 3) & 15;
-        for (int r = col - ((col + at) & 15) + l16; r < n; r += kB) {
-            if (r < col) continue;
-            double const x = fix64::entry_to_double(
-                fix64::join(fix64::unpack(P[block_at(r / kB, J) + col % kB * kS + r % kB])), scale[r] - 61);
-            int const first_nan = (bad[r] & fix64::kOutOfRange) ? 0 : fail;
-            l[r] = col >= first_nan ? __longlong_as_double(0x7ff8000000000000ll) : x;
-        }
+        for (int r = col - ((col + at) & 15) + l16; r < n; r += kB)
+            if (r >= col)
+                l[r] = fix64::entry_to_double(fix64::join(fix64::unpack(P[block_at(r / kB, J) + col % kB * kS + r % kB])),
+                                              scale[r] - 61);
     }
 }
 
 template <bool SOLVE, bool HOST, class Batch>
-__global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t count, int N, int32_t* info) {
+__global__ void __launch_bounds__(32, 8) posv_pair_kernel(Batch batch, int64_t count, int N, int32_t* info) {
     extern __shared__ __align__(16) unsigned char smem[];
     int const l16 = threadIdx.x & 15, half = threadIdx.x >> 4;
     Layout const lay = layout_of(N);
@@ -361,7 +411,7 @@ __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t 
     int64_t* P = reinterpret_cast<int64_t*>(base);
     Rsqrt* rsq = reinterpret_cast<Rsqrt*>(base + lay.rsqrt);
     int* scale = reinterpret_cast<int*>(base + lay.scale);
-    unsigned char* bad = base + lay.bad;
+    uint32_t* row = reinterpret_cast<uint32_t*>(base + lay.row);
     int64_t const b = 2 * (int64_t)blockIdx.x + half;
     PairItem it;
     it.n = 0, it.nrhs = 0;
@@ -400,66 +450,76 @@ __global__ void __launch_bounds__(32, 12) posv_pair_kernel(Batch batch, int64_t 
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncwarp();
+    bool sound = true;  // of this matrix, as far as this lane has seen
     for (int i = l16; i < kB * blocks; i += kB) {
         int e = 0;
-        bool ok = true;
-        int const J = i / kB;
-        if (i < n)
-            ok = fix64::scale_exponent(
-                __longlong_as_double(P[block_at(J, J) + (i - kB * J) * (kS + 1)]), e);
+        if (i < n) sound &= fix64::scale_exponent(__longlong_as_double(P[block_at(i / kB, i / kB) + i % kB * (kS + 1)]), e);
         scale[i] = e;
-        bad[i] = ok ? 0 : fix64::kNoPivot;
+        row[i] = 0;
     }
-    __syncwarp();
-    for (int i = l16; i < n; i += kB) {
-        if (bad[i]) {
-            int e = scale[i];
-            for (int j = 0; j < i; ++j) {
-                double const a = __longlong_as_double(P[block_at(i / kB, j / kB) + j % kB * kS + i % kB]);
-                if (!bad[j]) e = max(e, fix64::exponent_of(a) - scale[j] + fix64::kGrowth);
-            }
-            scale[i] = e;
-        }
-    }
-    __syncwarp();
-    int fail = n;
-    for (int J = 0; J < blocks; ++J) {
+    unsigned const half_mask = 0xffffu << (16 * half);
+    uint32_t const below = fix64::weak_below(n);
+    // The first block column that is left to binary64.
+    int redo = (__ballot_sync(0xffffffffu, !sound) & half_mask) ? 0 : blocks;
+    for (int J = 0; J < blocks && __any_sync(0xffffffffu, n > 0 && redo == blocks); ++J) {
         for (int I = J; I < blocks; ++I) {
             int const rows = nmax - kB * I;  // only the last block can have fewer than 16
-            if (rows <= 4) block_remainder<1>(P, n, I, J, scale, bad, l16 & 3, l16 >> 2);
-            else if (rows <= 8) block_remainder<2>(P, n, I, J, scale, bad, l16 & 3, l16 >> 2);
-            else block_remainder<4>(P, n, I, J, scale, bad, l16 & 3, l16 >> 2);
+            if (rows <= 4) sound &= block_remainder<1>(P, n, I, J, scale, l16 & 3, l16 >> 2);
+            else if (rows <= 8) sound &= block_remainder<2>(P, n, I, J, scale, l16 & 3, l16 >> 2);
+            else sound &= block_remainder<4>(P, n, I, J, scale, l16 & 3, l16 >> 2);
         }
         __syncwarp();
-        factor_diagonal(P + block_at(J, J), kB * J, min(kB, nmax - kB * J), rsq, bad + kB * J, l16, fail);
+        auto look = [&](int first, unsigned weak) {
+            __syncwarp();
+            if (first + l16 >= n || redo != blocks) weak = 0;
+            if (__any_sync(0xffffffffu, weak != 0)) sound &= served(P, row, it.A, it.lda, n, first, J, below, weak, l16);
+        };
+        unsigned weak = 0;
+        sound &= factor_diagonal(P + block_at(J, J), n - kB * J, min(kB, nmax - kB * J), rsq, row[kB * J + l16], l16, below, weak);
+        look(kB * J, weak);
+        for (int I = J + 1; I < blocks; ++I) {
+            weak = 0;
+            sound &= solve_block_row(P + block_at(I, J) + l16, kB * I + l16 < nmax, P + block_at(J, J), rsq, row[kB * I + l16],
+                                     below, weak);
+            look(kB * I, weak);
+        }
         __syncwarp();
-        for (int I = J + 1; I < blocks; ++I)
-            if (!solve_block_row(P + block_at(I, J) + l16, kB * I + l16 < nmax, P + block_at(J, J), rsq)) bad[kB * I + l16] = fix64::kNoPivot | fix64::kOutOfRange;
-        __syncwarp();
-        if constexpr (HOST) store_columns(it, n, J, blocks, fail, P, scale, bad, l16);
+        if ((__ballot_sync(0xffffffffu, !sound) & half_mask) && redo == blocks) redo = J;
+        if constexpr (HOST)
+            if (redo == blocks) store_columns(it, n, J, P, scale, l16);
     }
-    if (info && l16 == 0 && have) info[b] = fail < n ? fail + 1 : 0;
-    // The factor to memory. After a pivot that is not positive the columns from it on are NaN, and so are
-    // the rows whose entries left the fixed-point range.
-    bool again = !HOST;  // in host memory already, but for rows found out of range since
-    if constexpr (HOST)
-        for (int i = l16; i < n; i += kB) again |= (bad[i] & fix64::kOutOfRange) != 0;
-    again = __any_sync(0xffffffffu, again);
-    for (int I = 0; I < (again || SOLVE ? blocks : 0); ++I) {
-        int const r = kB * I + l16, e = scale[r] - 61, first_nan = (bad[r] & fix64::kOutOfRange) ? 0 : fail;
-        for (int J = 0; J <= I; ++J) {
-            int64_t* blk = P + block_at(I, J) + l16;
-            double* l = it.L + r + (int64_t)(kB * J) * it.ldl;
+    // The factor becomes binary64 in place and goes to memory; block columns from redo on are read again.
+    int fail = 0;
+    if (SOLVE || !HOST || __any_sync(0xffffffffu, n > 0 && redo < blocks)) {
+        for (int I = 0; I < blocks; ++I) {
+            int const r = kB * I + l16, e = scale[r] - 61;
+            for (int J = 0; J <= I; ++J) {
+                int64_t* blk = P + block_at(I, J) + l16;
+                double* l = it.L + r + (int64_t)(kB * J) * it.ldl;
+                double const* a = it.A + r + (int64_t)(kB * J) * it.lda;
+                bool const again = J >= redo;
 #pragma unroll 4
-            for (int c = 0; c < kB; ++c) {
-                int const col = kB * J + c;
-                double x = fix64::entry_to_double(fix64::join(fix64::unpack(blk[c * kS])), e);
-                if (col >= first_nan) x = __longlong_as_double(0x7ff8000000000000ll);
-                if (SOLVE && col <= r) blk[c * kS] = r < n ? __double_as_longlong(x) : 0;
-                if (again && col <= r && r < n) l[c * it.ldl] = x;
+                for (int c = 0; c < kB; ++c) {
+                    if (kB * J + c > r) continue;
+                    double x = 0.0;
+                    if (r < n) x = again ? a[c * it.lda] : fix64::entry_to_double(fix64::join(fix64::unpack(blk[c * kS])), e);
+                    if (SOLVE || redo < blocks) blk[c * kS] = __double_as_longlong(x);
+                    if (!HOST && !again && r < n) l[c * it.ldl] = x;
+                }
             }
         }
+        if (redo < blocks && n > 0) {
+            double* F = reinterpret_cast<double*>(P);
+            auto at = [=](int r, int c) -> double& { return F[block_at(r / kB, c / kB) + c % kB * kS + r % kB]; };
+            auto sync = [=] { __syncwarp(half_mask); };
+            sync();
+            fail = potrf_strips<kB>(n, kB * redo, 0, at, at, [](int) { return true; }, reinterpret_cast<double*>(rsq), l16, sync);
+            for (int c = kB * redo; c < n; ++c)
+                for (int r = c / kB * kB + l16; r < n; r += kB)
+                    if (r >= c) it.L[r + (int64_t)c * it.ldl] = at(r, c);
+        }
     }
+    if (info && l16 == 0 && have) info[b] = fail;
     if constexpr (SOLVE) {
         double* F = reinterpret_cast<double*>(P);
         double* rd = reinterpret_cast<double*>(rsq);

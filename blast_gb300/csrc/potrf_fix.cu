@@ -23,6 +23,8 @@
 //  * The first chunk's first 32 rows: one warp, a row per lane, the 16 columns right-looking in
 //    registers, the pivot row's limbs by shuffles. The reciprocal square root is integer as well.
 //  * Other rows: a row per thread against the diagonal block, left-looking in registers.
+//  * A row of a panel that cannot be certified (fix64.cuh) is not stored. After its chunk the columns so far
+//    become binary64, and what is left of the matrix is factored in binary64 (potrf_strips.cuh).
 //  * The factor stays in fixed point in the workspace (L itself, unless the caller says otherwise), as
 //    limbs or as digits, where the later panels read it, and becomes binary64 in one last pass.
 //
@@ -30,6 +32,7 @@
 // products, and let all T threads own a row of it.
 #include "common.cuh"
 #include "fix64.cuh"
+#include "potrf_strips.cuh"
 
 namespace blastgpu {
 namespace {
@@ -54,8 +57,8 @@ struct Shape {
     static constexpr int kDiag = kChunk + kNB * CS * 8;
     static constexpr int kRsqrt = kDiag + kNB * kNB * 8;
     static constexpr int kScale = kRsqrt + kNB * 16;
-    static constexpr int kBad = kScale + NMAX * 4;
-    static constexpr int kBytes = kBad + NMAX;
+    static constexpr int kRow = kScale + NMAX * 2;
+    static constexpr int kBytes = kRow + NMAX * 4;
 };
 
 template <int T>
@@ -119,8 +122,8 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t const (&a)[4], u
 // are not used.
 template <int T, int RA>
 __device__ __forceinline__ void update_chunk_int(int k0, int r0, int mr, int nb, const double* A, int64_t lda,
-                                             const int64_t* W, int64_t ldw, int64_t* stage, int64_t* C, const int* scale,
-                                             unsigned char* bad) {
+                                             const int64_t* W, int64_t ldw, int64_t* stage, int64_t* C, const short* scale,
+                                             uint32_t* row) {
     using S = Shape<T>;
     int const lane = threadIdx.x & 31, ct = 4 * (lane >> 3), rt = 8 * (threadIdx.x >> 5) + (lane & 7);
     int const slabs = k0 / kNB;
@@ -147,7 +150,7 @@ __device__ __forceinline__ void update_chunk_int(int k0, int r0, int mr, int nb,
             hh[i][j] = -v;
             cr[i][j] = fix64::kCrossStart;
         }
-        if (!ok && r < mr) bad[k0 + r0 + r] = fix64::kNoPivot | fix64::kOutOfRange;
+        if (!ok && r < mr) atomicOr(row + k0 + r0 + r, fix64::kTodo);
     }
     int64_t const* colbase = stage + (r0 == 0 ? ct : T + ct);
     int64_t const* rowbase = stage + rt;
@@ -205,7 +208,7 @@ __device__ __forceinline__ void update_chunk_int(int k0, int r0, int mr, int nb,
 template <int T>
 __device__ __forceinline__ void update_chunk_mma(int k0, int r0, int mr, int nb, const double* A, int64_t lda,
                                                  const int64_t* W, int64_t ldw, int64_t* stage, uint4* digits, int64_t* C,
-                                                 const int* scale, unsigned char* bad) {
+                                                 const short* scale, uint32_t* row) {
     using S = Shape<T>;
     int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q2 = 2 * (lane & 3);
     {  // A's entries start towards L2: a column's 128-byte line per thread
@@ -308,43 +311,157 @@ __device__ __forceinline__ void update_chunk_mma(int k0, int r0, int mr, int nb,
                             ok &= fix64::from_double(A[(k0 + r0 + r) + (int64_t)(k0 + c) * lda], er + scale[k0 + c], v);
                         C[c * S::CS + r] = v - sum[t][n][2 * h + e];
                     }
-                if (!ok) bad[k0 + r0 + r] = fix64::kNoPivot | fix64::kOutOfRange;
+                if (!ok) atomicOr(row + k0 + r0 + r, fix64::kTodo);
             }
         }
 }
 
-// The panel's first 32 rows (mr of them exist), one warp, a row per lane: the 16 columns right-looking.
-// Leaves the diagonal block's entries in D, the pivots' reciprocal square roots in rsq, the entries
-// in W. Returns the number of columns factored (nb unless a pivot is not positive).
+// An entry of the workspace.
 template <int T>
-__device__ __forceinline__ int factor_diagonal(int k0, int mr, int nb, const int64_t* C, int64_t* W, int64_t ldw, Limbs* D,
-                                               Rsqrt* rsq, unsigned char* bad) {
+__device__ __forceinline__ int64_t to_workspace(int64_t q) {
+    return Shape<T>::kTensor ? fix64::to_digits(q) : fix64::pack(fix64::split(q));
+}
+template <int T>
+__device__ __forceinline__ int64_t from_workspace(int64_t w) {
+    return Shape<T>::kTensor ? fix64::from_digits(w) : fix64::join(fix64::unpack(w));
+}
+
+// Why the panels end early: a row, or the whole panel, is left to binary64.
+constexpr int kStopRow = 1, kStopPanel = 2;
+
+struct Panel {
+    int k0, nb;
+    const double* A;
+    int64_t lda;
+    int64_t* W;
+    int64_t ldw;
+    const Limbs* D;  // the diagonal block, row by row
+    uint32_t* row;   // the rows' words
+    uint32_t below;  // fix64::weak_below
+    int* stop;
+};
+
+// Whether the weak entries of the warp's rows first + lane of the panel are served by fixed point all the same
+// (fix64.cuh). C: the chunk's columns at row `first`, with the entries of the rows that have weak ones. The warp
+// looks at one entry at a time.
+template <int T>
+__device__ __noinline__ bool served(int first, int nb, int k0, const int64_t* C, const Limbs* D, const int64_t* W, int64_t ldw,
+                                    const double* A, int64_t lda, const uint32_t* words, uint32_t below, unsigned weak) {
     using S = Shape<T>;
     int const lane = threadIdx.x & 31;
+    bool ok = true;
+    for (;;) {
+        unsigned const who = __ballot_sync(0xffffffffu, weak != 0);
+        if (who == 0) return ok;
+        int const src = __ffs(who) - 1, i = first + src, j = __ffs(__shfl_sync(0xffffffffu, weak, src)) - 1;
+        bool through = false, term = false;
+        if (lane < nb && lane != i && lane != j) {
+            int const k = lane;
+            Limbs const u = k < i ? fix64::split(C[k * S::CS + src]) : D[k * kNB + i];
+            Limbs const v = D[max(j, k) * kNB + min(j, k)];
+            through = fix64::strong(u.h, v.h, below);
+            term = k < j && (u.h | u.l) != 0 && (v.h | v.l) != 0;
+        }
+        int const before = (words[i] & words[j] & fix64::kSeen) ? k0 : 0;
+        for (int k = lane; !__any_sync(0xffffffffu, through) && k - lane < before; k += 32) {
+            if (k < before) {
+                int64_t const u = from_workspace<T>(W[i + k * ldw]), v = from_workspace<T>(W[j + k * ldw]);
+                through = fix64::strong(fix64::high_limb(u), fix64::high_limb(v), below);
+                term |= u != 0 && v != 0;
+            }
+        }
+        // an entry of zero without terms is exact
+        bool const fine = __any_sync(0xffffffffu, through) ||
+                          !(__any_sync(0xffffffffu, term) || C[j * S::CS + src] != 0 || A[i + j * lda] != 0.0);
+        if (lane == src) {
+            ok = fine;
+            weak = ok ? weak & (weak - 1) : 0;
+        }
+    }
+}
+
+// Whether the warp's rows first + lane of the panel (mine: the lane has one) are certified; their words after the
+// panel. C: the chunk's columns at row `first`; q: the row's entries.
+template <int T>
+__device__ __forceinline__ bool certify(Panel const& p, int first, bool mine, const int64_t (&q)[kNB], int64_t* C, bool ok,
+                                        unsigned weak, int64_t squares, int any) {
+    int const lane = threadIdx.x & 31;
+    if (mine) {
+        uint32_t* const word = p.row + p.k0 + first + lane;
+        uint32_t const w = *word, now = (w + fix64::norm_of(squares)) | (any != 0 ? fix64::kSeen : 0);
+        ok &= (w & fix64::kTodo) == 0 && (now & fix64::kNormMask) <= fix64::kNormMost;
+        *word = now;
+        if ((now & fix64::kSeen) == 0)  // a row without any entry so far
+            for (; weak != 0; weak &= weak - 1)
+                ok &= p.A[p.k0 + first + lane + (p.k0 + __ffs(weak) - 1) * p.lda] == 0.0;
+    }
+    if (!mine || !ok) weak = 0;
+    if (__any_sync(0xffffffffu, weak != 0)) {
+        if (weak != 0) {
+#pragma unroll
+            for (int j = 0; j < kNB; ++j) C[j * Shape<T>::CS + lane] = q[j];
+        }
+        __syncwarp();
+        ok &= served<T>(first, p.nb, p.k0, C, p.D, p.W + p.k0, p.ldw, p.A + p.k0 + p.k0 * p.lda, p.lda, p.row + p.k0, p.below, weak);
+    }
+    return ok;
+}
+
+// A row that was taken through the panel: stored if it is certified, else left to binary64.
+template <int T>
+__device__ __forceinline__ void finish_row(Panel const& p, int i, int entries, const int64_t (&q)[kNB], bool ok) {
+    if (ok) {
+        int64_t* w = p.W + p.k0 + i + p.k0 * p.ldw;
+#pragma unroll
+        for (int j = 0; j < kNB; ++j)
+            if (j < entries) w[j * p.ldw] = to_workspace<T>(q[j]);
+    } else {
+        p.row[p.k0 + i] |= fix64::kTodo;
+        *p.stop = kStopRow;
+    }
+}
+
+// The panel's first 32 rows (mr of them exist), one warp, a row per lane: the 16 columns right-looking.
+// Leaves the diagonal block's entries in D and the pivots' reciprocal square roots in rsq.
+template <int T>
+__device__ __forceinline__ void factor_diagonal(Panel const& p, int mr, int64_t* C, Limbs* D, Rsqrt* rsq) {
+    using S = Shape<T>;
+    int const lane = threadIdx.x & 31, nb = p.nb;
     bool const mine = lane < mr;
-    int64_t acc[kNB], cr[kNB];
+    int64_t acc[kNB], cr[kNB];  // acc: column j's entry q once it is there
 #pragma unroll
     for (int c = 0; c < kNB; ++c) {
         acc[c] = mine && c < nb ? C[c * S::CS + lane] : 0;
         cr[c] = fix64::kCrossStart;
     }
-    bool const no_pivot = mine && bad[k0 + lane] != 0;
-    bool off = false;
-    int done = nb;
+    bool good = true, ok = true;
+    unsigned weak = 0;
+    int64_t squares = 0;
+    int any = 0;
     // The next pivot's reciprocal square root is taken as soon as its column is up to date, beside the
     // products of the columns after it.
-    int64_t t = acc[0] - fix64::total(0, cr[0]);
-    int64_t s = __shfl_sync(0xffffffffu, no_pivot ? (int64_t)-1 : t, 0);
-    if (s < fix64::kPivotMin) done = 0;
-    Rsqrt y = fix64::pivot_rsqrt(max(s, fix64::kPivotMin));
+    int64_t t = 0;
+    Rsqrt y;
+    auto pivot = [&](int c) {
+        t = acc[c] - fix64::total(0, cr[c]);
+        int64_t const s = __shfl_sync(0xffffffffu, t, c);
+        good &= s >= fix64::kPivotMin;
+        y = fix64::pivot_rsqrt(max(s, fix64::kPivotMin));
+    };
+    pivot(0);
 #pragma unroll
     for (int j = 0; j < kNB; ++j) {
-        if (j < done) {  // warp-uniform
+        if (j < nb) {  // warp-uniform
             int64_t q;
-            bool const ok = fix64::scale_entry(t, y, q);
-            off |= !ok && lane > j;
+            bool const in = fix64::scale_entry(t, y, q);
             Limbs const v = fix64::split(q);
-            if (lane >= j && mine) W[(k0 + lane) + (int64_t)(k0 + j) * ldw] = S::kTensor ? fix64::to_digits(q) : fix64::pack(v);
+            acc[j] = q;
+            if (fix64::weak(t, p.below)) weak |= 1u << j;
+            if (lane >= j) {
+                ok &= in;
+                fix64::add_square(squares, v.h);
+                any |= v.h | v.l;
+            }
             if (lane < kNB) D[lane * kNB + j] = v;
             if (lane == 0) rsq[j] = y;
 #pragma unroll
@@ -353,29 +470,34 @@ __device__ __forceinline__ int factor_diagonal(int k0, int mr, int nb, const int
                 fix64::mad(acc[c], -v.h, h);
                 fix64::mad(cr[c], v.h, l);
                 fix64::mad(cr[c], v.l, h);
-                if (c == j + 1 && c < nb) {
-                    t = acc[c] - fix64::total(0, cr[c]);
-                    s = __shfl_sync(0xffffffffu, off || no_pivot ? (int64_t)-1 : t, c);
-                    if (s < fix64::kPivotMin) done = c;
-                    y = fix64::pivot_rsqrt(max(s, fix64::kPivotMin));
-                }
+                if (c == j + 1 && c < nb) pivot(c);
             }
         }
     }
-    // Pivots that were not reached: rows are still solved against the columns before them.
-    for (int j = done + lane; j < kNB; j += 32) rsq[j] = y;
-    if (off) bad[k0 + lane] = fix64::kNoPivot | fix64::kOutOfRange;
-    return done;
+    weak &= lane < kNB ? (1u << lane) - 1 : 0xffffu;
+    __syncwarp();
+    // The diagonal block's rows are certified before any row is stored.
+    ok = certify<T>(p, 0, mine, acc, C, ok, weak, squares, any);
+    if (__all_sync(0xffffffffu, good && (ok || lane >= nb || !mine))) {
+        if (mine) finish_row<T>(p, lane, min(lane + 1, kNB), acc, ok);
+    } else if (lane == 0) {
+        *p.stop = kStopPanel;
+    }
 }
 
-// Row r of the chunk against the diagonal block, one thread. The columns past the first `done` are computed
-// from whatever D holds there, so that nothing branches between the columns, and not stored.
+// A warp's rows first + lane of the panel, r = r0 + lane of the chunk (mine: the lane has one), against the diagonal
+// block.
 template <int T>
-__device__ __forceinline__ void solve_row(int row, int r, int k0, int done, const int64_t* C, int64_t* W, int64_t ldw,
-                                          const Limbs* D, const Rsqrt* rsq, unsigned char* bad) {
+__device__ __forceinline__ void solve_rows(Panel const& p, int first, int r0, bool mine, int64_t* C, const Limbs* D,
+                                           const Rsqrt* rsq) {
     using S = Shape<T>;
+    int const r = r0 + (threadIdx.x & 31);
     Limbs x[kNB];
+    int64_t v[kNB];
     bool ok = true;
+    unsigned weak = 0;
+    int64_t squares = 0;
+    int any = 0;
 #pragma unroll
     for (int j = 0; j < kNB; ++j) {
         int64_t hh = 0, c0 = fix64::kCrossStart, c1 = 0;
@@ -387,15 +509,16 @@ __device__ __forceinline__ void solve_row(int row, int r, int k0, int done, cons
             fix64::mad(c1, x[q].l, d.h);
         }
         int64_t const t = C[j * S::CS + r] - fix64::total(hh, c0 + c1);
-        int64_t v;
-        bool const in = fix64::scale_entry(t, rsq[j], v);
-        x[j] = fix64::split(v);
-        if (j < done) {
-            ok &= in;
-            W[row + (int64_t)(k0 + j) * ldw] = S::kTensor ? fix64::to_digits(v) : fix64::pack(x[j]);
-        }
+        ok &= fix64::scale_entry(t, rsq[j], v[j]);
+        if (fix64::weak(t, p.below)) weak |= 1u << j;
+        x[j] = fix64::split(v[j]);
+        fix64::add_square(squares, x[j].h);
+        any |= x[j].h | x[j].l;
     }
-    if (!ok) bad[row] = fix64::kNoPivot | fix64::kOutOfRange;
+#pragma unroll
+    for (int j = 0; j < kNB; ++j) v[j] = fix64::join(x[j]);
+    ok = certify<T>(p, first, mine, v, C + r0, ok, weak, squares, any);
+    if (mine) finish_row<T>(p, first + (threadIdx.x & 31), kNB, v, ok);
 }
 
 // One matrix. W: the fixed-point factor while the matrix is being factored, n rows of 8 bytes per
@@ -413,7 +536,7 @@ struct FixItem {
 };
 
 template <int T, class Batch>
-__global__ void __launch_bounds__(T, T == 128 ? 3 : 512 / T) potrf_fix_kernel(Batch batch, int32_t* info) {
+__global__ void __launch_bounds__(T, T == 128 ? 3 : T == 64 ? 7 : 11) potrf_fix_kernel(Batch batch, int32_t* info) {
     using S = Shape<T>;
     extern __shared__ __align__(16) unsigned char smem[];
     int64_t* stage = reinterpret_cast<int64_t*>(smem + S::kStage);
@@ -421,40 +544,35 @@ __global__ void __launch_bounds__(T, T == 128 ? 3 : 512 / T) potrf_fix_kernel(Ba
     int64_t* C = reinterpret_cast<int64_t*>(smem + S::kChunk);
     Limbs* D = reinterpret_cast<Limbs*>(smem + S::kDiag);
     Rsqrt* rsq = reinterpret_cast<Rsqrt*>(smem + S::kRsqrt);
-    int* scale = reinterpret_cast<int*>(smem + S::kScale);
-    unsigned char* bad = smem + S::kBad;
-    __shared__ int s_done;
+    short* scale = reinterpret_cast<short*>(smem + S::kScale);
+    uint32_t* row = reinterpret_cast<uint32_t*>(smem + S::kRow);
+    __shared__ int s_stop;
     int64_t const b = blockIdx.x;
     FixItem it;
     if (!batch.get(b, it) || it.n > S::NMAX) return;
     int const n = it.n, tid = threadIdx.x;
     int64_t* W = reinterpret_cast<int64_t*>(it.W);
+    if (tid == 0) s_stop = 0;
+    cta_sync<T>();
     for (int i = tid; i < n; i += T) {
         int e;
-        bad[i] = fix64::scale_exponent(it.A[i + (int64_t)i * it.lda], e) ? 0 : fix64::kNoPivot;
-        scale[i] = e;
+        if (!fix64::scale_exponent(it.A[i + (int64_t)i * it.lda], e)) s_stop = kStopPanel;
+        scale[i] = (short)e;
+        row[i] = 0;
     }
     cta_sync<T>();
-    for (int i = tid; i < n; i += T) {
-        if (bad[i]) {
-            int e = scale[i];
-            for (int j = 0; j < i; ++j)
-                if (!bad[j]) e = max(e, fix64::exponent_of(it.A[i + (int64_t)j * it.lda]) - scale[j] + fix64::kGrowth);
-            scale[i] = e;
-        }
-    }
-    cta_sync<T>();
-    int good = n;  // columns factored
-    for (int k0 = 0; k0 < n; k0 += kNB) {
+    uint32_t const below = fix64::weak_below(n);
+    int stop = s_stop, k0 = 0, r0 = 0;
+    for (; k0 < n && stop == 0; k0 += stop == 0 ? kNB : 0) {
         int const nb = min(kNB, n - k0), m = n - k0;
-        int done = nb;
-        for (int r0 = 0; r0 < m; r0 += T) {
+        Panel const p{k0, nb, it.A, it.lda, W, it.ldw, D, row, below, &s_stop};
+        for (r0 = 0; r0 < m && stop == 0; r0 += stop == 0 ? T : 0) {
             int const mr = min(T, m - r0);
             if constexpr (S::kTensor) {
-                update_chunk_mma<T>(k0, r0, mr, nb, it.A, it.lda, W, it.ldw, stage, digits, C, scale, bad);
+                update_chunk_mma<T>(k0, r0, mr, nb, it.A, it.lda, W, it.ldw, stage, digits, C, scale, row);
             } else {
 #define BLASTGPU_UPDATE(RA) \
-    update_chunk_int<T, RA>(k0, r0, mr, nb, it.A, it.lda, W, it.ldw, stage, C, scale, bad)
+    update_chunk_int<T, RA>(k0, r0, mr, nb, it.A, it.lda, W, it.ldw, stage, C, scale, row)
                 switch ((mr + S::RT - 1) / S::RT) {
                     case 1: BLASTGPU_UPDATE(1); break;
                     case 2: BLASTGPU_UPDATE(2); break;
@@ -465,28 +583,22 @@ __global__ void __launch_bounds__(T, T == 128 ? 3 : 512 / T) potrf_fix_kernel(Ba
             }
             cta_sync<T>();
             if (r0 == 0) {
-                if (tid < 32) {
-                    done = factor_diagonal<T>(k0, mr, nb, C, W, it.ldw, D, rsq, bad);
-                    if (tid == 0) s_done = done;
-                }
+                if (tid < 32) factor_diagonal<T>(p, mr, C, D, rsq);
                 cta_sync<T>();
-                done = s_done;
             }
-            if (tid < mr && (r0 > 0 || tid >= 32))
-                solve_row<T>(k0 + r0 + tid, tid, k0, done, C, W, it.ldw, D, rsq, bad);
+            // Nobody writes kStopPanel from here on, so every thread sees the same side of it.
+            int const warp_row = tid & ~31;
+            if (s_stop != kStopPanel && warp_row < mr && (r0 > 0 || warp_row > 0))
+                solve_rows<T>(p, r0 + warp_row, warp_row, tid < mr, C, D, rsq);
             cta_sync<T>();  // C is written again; the panel's columns are read from now on
-        }
-        if (done < nb) {
-            good = k0 + done;
-            break;
+            stop = s_stop;  // not written again before the next chunk's barriers
         }
     }
-    if (info && tid == 0) info[b] = good < n ? good + 1 : 0;
-    // Fixed point to binary64, a warp per column. After a pivot that is not positive the columns from it
-    // on are NaN, and so are the rows whose entries left the fixed-point range.
-    double const nan = __longlong_as_double(0x7ff8000000000000ll);
+    // Fixed point to binary64, a warp per column: all of it, or what was certified.
+    int const whole = stop == 0 ? n : k0, columns = stop == kStopRow ? k0 + kNB : whole;
+    auto todo = [=](int i) { return i >= k0 + r0 + T || (row[i] & fix64::kTodo) != 0; };  // in columns whole .. columns-1
     int const lane = tid & 31, warp = tid >> 5;
-    for (int c = warp; c < n; c += T / 32) {
+    for (int c = warp; c < columns; c += T / 32) {
         int64_t const* w = W + (int64_t)c * it.ldw;
         double* l = it.L + (int64_t)c * it.ldl;
         for (int i0 = c; i0 < n; i0 += 128) {
@@ -494,21 +606,32 @@ __global__ void __launch_bounds__(T, T == 128 ? 3 : 512 / T) potrf_fix_kernel(Ba
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 int const i = i0 + lane + 32 * u;
-                v[u] = i < n && c < good ? w[i] : 0;
+                v[u] = i < n ? w[i] : 0;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 int const i = i0 + lane + 32 * u;
-                if (i < n) {
-                    int64_t const q = S::kTensor ? fix64::from_digits(v[u]) : fix64::join(fix64::unpack(v[u]));
-                    double x = fix64::entry_to_double(q, scale[i] - 61);
-                    if (c >= good || (bad[i] & fix64::kOutOfRange)) x = nan;
+                if (i < n && (c < whole || !todo(i))) {
+                    double const x = fix64::entry_to_double(from_workspace<T>(v[u]), scale[i] - 61);
                     l[i] = x;
                     if (it.L2) it.L2[i + (int64_t)c * it.ldl2] = x;
                 }
             }
         }
     }
+    int fail = 0;
+    if (stop != 0) {
+        double* F = it.L2 ? it.L2 : it.L;
+        int64_t const ldf = it.L2 ? it.ldl2 : it.ldl;
+        auto sync = [] { cta_sync<T>(); };
+        sync();
+        fail = potrf_strips<T>(n, whole, columns, [=](int r, int c) { return it.A[r + c * it.lda]; },
+                               [=](int r, int c) -> double& { return F[r + c * ldf]; }, todo,
+                               reinterpret_cast<double*>(rsq), tid, sync);
+        for (int c = whole + warp; c < n && it.L2; c += T / 32)
+            for (int i = c + lane; i < n; i += 32) it.L[i + (int64_t)c * it.ldl] = it.L2[i + (int64_t)c * it.ldl2];
+    }
+    if (info && tid == 0) info[b] = fail;
 }
 
 struct FixStrided {

@@ -130,3 +130,123 @@ def test_non_finite_right_hand_sides(gpu, oracle_lib, n):
     want = oracle_lib.posv_batch(A[None], B[None])[1][0]
     assert np.array_equal(np.isfinite(X[0]), np.isfinite(want)) and X[0][n - 1, 2] == np.inf
     check(A, B[:, :1], X[0][:, :1])
+
+
+def coupled(n):
+    """Matrices whose unknowns are coupled weakly, directly or by way of many others: entries of the matrix, of its
+    factor and of the solution fall far below their rows' largest."""
+    rng = np.random.default_rng(n)
+    i, h = np.arange(n), n // 2
+    d = np.abs(i[:, None] - i[None, :])
+    blocks = np.zeros((n, n))
+    blocks[:h, :h], blocks[h:, h:] = spd(rng, h), spd(rng, n - h)
+    for entry in (1e-20, 1e-9):
+        A = blocks.copy()
+        A[n - 2, 3] = A[3, n - 2] = entry
+        yield A
+    A = blocks.copy()
+    A[h:, :h] = 1e-7 * rng.standard_normal((n - h, h))
+    A[:h, h:] = A[h:, :h].T
+    yield A
+    yield np.exp(-(0.9 * d) ** 2 / 2) + 0.1 * np.eye(n)  # a Gaussian kernel
+    yield np.exp(-3.0 * d)
+    A = 4.0 * np.eye(n) - (d == 1) - (d == n - 1)  # a ring
+    yield A
+    yield A * np.outer(2.0 ** (i % 5 * 20), 2.0 ** (i % 5 * 20))
+
+
+@pytest.mark.parametrize("n", [17, 33, 48, 64, 65, 129, 200])
+def test_weakly_coupled_unknowns(gpu, n):
+    import torch
+
+    As = list(coupled(n))
+    B = np.stack([np.eye(n)[0], np.eye(n)[n - 1], np.eye(n)[n // 2], np.random.default_rng(n).standard_normal(n)], 1)
+    info, L, X = run(gpu, As, [B] * len(As))
+    assert not info.any()
+    for A, l, x in zip(As, L, X):
+        check(A, B, x, l)
+    P = to_dev(np.stack(As))  # in place
+    info2 = gpu.potrf(P, P)
+    torch.cuda.synchronize()
+    assert not info2.any() and np.array_equal(np.tril(P.cpu().numpy()), np.tril(L))
+
+
+@pytest.mark.parametrize("ns", [[17, 40, 64, 33], [20, 128, 65, 48], [300, 129, 18, 100]])
+def test_weakly_coupled_ragged(gpu, ns):
+    """The same through the ragged plan, and with the factor taken again in the adjoint."""
+    import torch
+
+    from blast_gb300.autograd import spd_solve_packed
+    from blast_gb300.ragged import Packed, PosvPlan
+
+    which = [(n, k) for n in ns if n <= 129 for k in range(7)] + [(n, 5) for n in ns if n > 129]
+    As = [list(coupled(n))[k] for n, k in which]
+    n = [a for a, _ in which]
+    Bs = [np.eye(a)[:, :1] + (np.arange(a) == a - 1)[:, None] for a in n]
+    A, B, X, L = (Packed(n, c, "cuda") for c in (n, [1] * len(n), [1] * len(n), n))
+    A.fill_from(As)
+    B.fill_from(Bs)
+    plan = PosvPlan(A, B, X, L)
+    plan.run()
+    a, b = A.buf.clone().requires_grad_(), B.buf.clone().requires_grad_()
+    spd_solve_packed(a, b, np.array(n), np.ones(len(n), dtype=np.int64), keep_factor=False).backward(B.buf)
+    torch.cuda.synchronize()
+    assert not plan.results()[0].any()
+    at = 0
+    for m, Ah, Bh, Lg, Xg in zip(n, As, Bs, L.to_list(), X.to_list()):
+        check(Ah, Bh, Xg, Lg)
+        check(Ah, Bh, b.grad[at:at + m].cpu().numpy()[:, None])
+        at += m
+
+
+@pytest.mark.parametrize("n", [65, 80, 150])
+def test_weakly_coupled_mirror(gpu, n):
+    """The entry for host memory: the device call's factor, with workspaces of its own."""
+    import torch
+
+    from blast_gb300 import _lib
+
+    As = np.stack(list(coupled(n)))
+    m = len(As)
+    dA, dB = to_dev(As), to_dev(np.tile(np.eye(n)[:, :1], (m, 1, 1)))
+    L, X = gpu.col_major((m,), n, n, "cuda").zero_(), gpu.col_major((m,), n, 1, "cuda")
+    gpu.posv(dA, L, dB, X)
+    hL, hX = torch.zeros(m * n * n).double().pin_memory(), torch.zeros(m * n).double().pin_memory()
+    wL, wX = torch.empty(m * n * n, device="cuda").double(), torch.empty(m * n, device="cuda").double()
+    info = torch.full((m,), -1, dtype=torch.int32, device="cuda")
+    _lib.call("blastgpu_dposv_mirror_strided", n, 1, dA.data_ptr(), n, n * n, dB.data_ptr(), n, n, hL.data_ptr(), n, n * n,
+              hX.data_ptr(), n, n, wL.data_ptr(), wX.data_ptr(), info.data_ptr(), m, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert not info.any()
+    assert np.array_equal(np.tril(hL.numpy().reshape(m, n, n).transpose(0, 2, 1)), np.tril(L.cpu().numpy()))
+    for k in range(m):
+        check(As[k], np.eye(n)[:, :1], hX.numpy()[k * n:(k + 1) * n, None])
+
+
+@pytest.mark.parametrize("n", [17, 33, 64, 65, 128, 300, 512])
+def test_info_is_binary64s(gpu, oracle_lib, n):
+    """Pivots down to nothing, and rows far too long for their diagonal: info as binary64 finds it."""
+    import torch
+
+    As = []
+    for x in (2.0 ** -26 * np.sqrt(1 - 2.0 ** -10), 2.0 ** -26 * np.sqrt(1 - 2.0 ** -25), 2.0 ** -26):  # pivot 2^-62, 2^-77, 0
+        A = np.eye(n)
+        A[n - 1, n - 1] += 2.0 ** -52
+        A[n - 1, 0] = A[0, n - 1] = 1.0
+        A[n - 1, 1] = A[1, n - 1] = x
+        As.append(A)
+    for x in np.concatenate([np.linspace(0.1, 1.9999, 40), [1.99999]]):
+        A = np.eye(n)
+        A[n - 1, :n - 1] = A[:n - 1, n - 1] = x
+        As.append(A)
+    As = np.stack(As)
+    P = to_dev(As)
+    info = gpu.potrf(P, P)
+    torch.cuda.synchronize()
+    got = P.cpu().numpy()
+    for k, A in enumerate(As):
+        ref = np.zeros((n, n), order="F")
+        want = oracle_lib.potrf(np.asfortranarray(A), ref)
+        assert info[k] == want, (k, int(info[k]), want)
+        if want == 0:
+            assert np.allclose(np.tril(got[k]), np.tril(ref), rtol=10 * n * EPS, atol=0)
