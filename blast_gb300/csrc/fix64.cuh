@@ -27,10 +27,10 @@
 // binary64's follows them down. Where unknowns are coupled weakly (a kernel's far points, blocks with a
 // small entry between them), the solution's small entries come from such small terms. So the kernels
 // certify what they factor here, panel by panel, and leave the rest of a matrix to binary64 where
-//  * an entry's terms |l_ik l_jk| are all below a threshold, the last one, |l_ij l_jj|, among them (weak()),
-//    and i and j are not both coupled to another unknown of the panel with |l_ik l_kj| above it either,
-//    through which binary64's errors reach the same unknowns. An entry of zero with no term at all is exact.
-//    The threshold is 2^-16 at n = 17 and falls with n, so that the error is at most about 10 n 2^-52 of the
+//  * an entry is weak, |l_ij l_jj| below a threshold (weak()), and so is the sum of its other terms |l_ik l_jk|,
+//    together with |l_ik l_kj| over the panel's other unknowns, through which i and j are coupled and
+//    binary64's errors reach the same unknowns. An entry of zero with no term at all is exact. The
+//    threshold is 2^-16 at n = 17 and falls with n, so that the error is at most about 10 n 2^-52 of the
 //    terms (weak_shift()). Gaussian and Riccati matrices have no such entry in thousands, and one or two
 //    weak entries to look at from n = 48 on;
 //  * a pivot is below 2^-42 of its diagonal entry or so (kPivotMin): whether it is positive is then for
@@ -108,10 +108,53 @@ FIX64_FN void mad(int64_t& a, int32_t x, int32_t y) {
 #endif
 }
 
+// d = c + x * y.
+FIX64_FN void mad_to(int64_t& d, int64_t c, int32_t x, int32_t y) {
+#ifdef __CUDA_ARCH__
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(x), "r"(y), "l"(c));
+#else
+    d = c + (int64_t)x * y;
+#endif
+}
+
 FIX64_FN Limbs split(int64_t q) {
     int32_t const h = (int32_t)((q + (int64_t(1) << 29)) >> 30);
     return {(int32_t)(lo32(q) - ((uint32_t)h << 30)), h};
 }
+
+// Sums of a triangle of 16 columns that a row is taken through, column by column: sum[u], cross[u] belong to the u-th
+// column from the one at hand. The remainder of the first, once it is up to date:
+FIX64_FN int64_t remainder_of(int64_t sum, int64_t cross) { return sum - ((-cross) >> 30); }
+constexpr int64_t kCrossOfRemainder = -(int64_t(1) << 29);
+// Takes the product of the entry v of the column at hand with d off column u and moves its sums on.
+template <int N>
+FIX64_FN void take_off(int64_t (&sum)[N], int64_t (&cross)[N], int u, Limbs v, Limbs d) {
+    mad_to(sum[u - 1], sum[u], -v.h, d.h);
+    mad_to(cross[u - 1], cross[u], -v.h, d.l);
+    mad(cross[u - 1], -v.l, d.h);
+}
+
+#ifdef __CUDACC__
+// Runs column() for the 16 columns of a triangle, up to `cols` of them: its argument is how many columns are left, as a
+// type, rounded up to 16, 12, 8 or 4. The four loops are not unrolled: all 16 columns one after another were 56 KB of
+// code, and the kernels' warps waited for the instruction cache.
+template <int LEFT>
+struct Left {
+    static constexpr int value = LEFT;
+};
+template <class Column>
+__device__ __forceinline__ void triangle(int cols, Column&& column) {
+    int j = 0;
+#pragma unroll 1
+    for (; j < min(4, cols); ++j) column(Left<16>{}, j);
+#pragma unroll 1
+    for (; j < min(8, cols); ++j) column(Left<12>{}, j);
+#pragma unroll 1
+    for (; j < min(12, cols); ++j) column(Left<8>{}, j);
+#pragma unroll 1
+    for (; j < min(16, cols); ++j) column(Left<4>{}, j);
+}
+#endif
 
 // The limbs' place in memory: 8 bytes, l first.
 FIX64_FN int64_t pack(Limbs v) { return (int64_t)((uint64_t)(uint32_t)v.h << 32 | (uint32_t)v.l); }
@@ -156,15 +199,15 @@ FIX64_FN bool scale_exponent(double aii, int& e) {
 
 // The threshold below which an entry is weak is 2^-(16 + weak_shift(n)): 2^-61 of error is 10 n 2^-52 of it, or less.
 FIX64_FN int weak_shift(int n) { return (n >= 34) + (n >= 68) + (n >= 136) + (n >= 272); }
-// Whether |t| is below it (t, an entry's remainder l_ij l_jj, in units of 2^-62; below: weak_below(n)).
+// The same in the high words of numbers in units of 2^-62.
 FIX64_FN uint32_t weak_below(int n) { return (uint32_t(1) << 14) >> weak_shift(n); }
+// Whether entry (i, j)'s remainder t = l_ij l_jj is below it.
 FIX64_FN bool weak(int64_t t, uint32_t below) { return (uint32_t)hi32(t) + below < 2 * below; }
-// Whether the product of two entries with these high limbs is above it.
-FIX64_FN bool strong(int32_t h1, int32_t h2, uint32_t below) {
+// The high word of the product of two entries with these high limbs.
+FIX64_FN uint32_t term(int32_t h1, int32_t h2) {
     uint64_t const a = (uint32_t)(h1 < 0 ? -h1 : h1), b = (uint32_t)(h2 < 0 ? -h2 : h2);
-    return (uint32_t)(a * b >> 32) >= below;
+    return (uint32_t)(a * b >> 32);
 }
-FIX64_FN int32_t high_limb(int64_t q) { return (int32_t)(q >> 30); }
 
 // Sum of squares of the high limbs of a row's entries in a panel: 16 of them fit 64 bits without a sign, and
 // norm_of makes units of 2^-26 of them.
@@ -172,9 +215,15 @@ FIX64_FN void add_square(int64_t& sum, int32_t h) { mad(sum, h, h); }
 FIX64_FN uint32_t norm_of(int64_t sum) { return (uint32_t)((uint64_t)sum >> 36); }
 // 1/4, and more than what rounding the limbs may add.
 constexpr uint32_t kNormMost = (uint32_t(1) << 24) + (uint32_t(1) << 10);
-// A row's word: the sum of squares, whether it has had an entry other than zero, and whether its entries
-// of the panel at hand are left to binary64.
-constexpr uint32_t kNormMask = (uint32_t(1) << 28) - 1, kSeen = uint32_t(1) << 28, kTodo = uint32_t(1) << 29;
+// A row's word: the sum of squares; whether its entries of the panel at hand are left to binary64; and its first
+// panel with an entry other than zero before the diagonal, or a later one. A new row's word, and the word after panel
+// J with these squares (any: there was such an entry).
+constexpr uint32_t kNormMask = (uint32_t(1) << 26) - 1, kTodo = uint32_t(1) << 26, kNewRow = uint32_t(31) << 27;
+FIX64_FN int first_panel(uint32_t word) { return (int)(word >> 27); }
+FIX64_FN uint32_t row_after(uint32_t word, int J, int64_t squares, bool any) {
+    uint32_t const norm = (word & kNormMask) + norm_of(squares), first = any && J < first_panel(word) ? (uint32_t)J : word >> 27;
+    return (norm < kNormMask ? norm : kNormMask) | (word & kTodo) | first << 27;
+}
 
 // a * 2^-scale in units of 2^-62 (scale = e_i + e_j), truncated. False if |a| * 2^-scale is not below
 // 1/4 (or a is not finite): the matrix is then not positive definite.

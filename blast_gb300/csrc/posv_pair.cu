@@ -4,12 +4,12 @@
 // Reference: blast::potrf (dense/Potrf.hpp:66-106), left-looking, and blast::trsm (dense/Trsm.hpp:17-66)
 // for the solves.
 //
-// What bounds it: integer instructions, 28,000 for two matrices of n = 48 without right-hand sides, a
-// quarter of them the products of block columns, and the chain of pivots, with 8 warps per SM; then the
-// solves' multiply-adds on the binary64 pipe. 50,000 matrices of n = 48 with 8 right-hand sides take 3.70 ms
-// (1.21 ms the factor alone, 1.78 with one right-hand side) against 4.15 ms for a binary64 thread per matrix;
-// 10,000 take a half, one matrix of n = 24 21 us a call instead of 53. A matrix has 16 lanes, so that the
-// work on the diagonal, which has 16 rows to share it, fills the warp with two matrices, and a batch of
+// What bounds it: integer instructions, 30,000 for two matrices of n = 48 without right-hand sides, a
+// quarter of them the products of block columns, the chain of pivots, with 8 warps per SM, and fetching
+// them (fix64::triangle); then the solves' multiply-adds on the binary64 pipe. 50,000 matrices of n = 48 with 8
+// right-hand sides take 3.42 ms (1.41 ms the factor alone) against 4.15 ms for a binary64 thread per
+// matrix; 10,000 take a half, one matrix of n = 24 23 us a call instead of 53. A matrix has 16 lanes, so that
+// the work on the diagonal, which has 16 rows to share it, fills the warp with two matrices, and a batch of
 // small matrices needs few warps. The matrix is read from memory once and written once; the earlier
 // columns, which a thread per matrix reads again for every strip, stay in shared memory.
 //
@@ -145,130 +145,118 @@ __device__ __forceinline__ bool block_remainder(int64_t* P, int n, int I, int J,
     return ok;
 }
 
-// A row's sum of squares and whether it has had an entry (fix64.cuh) after a panel; false if the sum is too large.
-__device__ __forceinline__ bool add_row(uint32_t& row, int64_t squares, int any) {
-    row = (row + fix64::norm_of(squares)) | (any != 0 ? fix64::kSeen : 0);
-    return (row & fix64::kNormMask) <= fix64::kNormMost;
-}
-
 // A diagonal block, a row per lane (16 lanes per matrix), right-looking. rows: rows of the block that the matrix
 // has; cols: columns that some matrix of the warp has. False if a pivot is too small, or the lane's row out of
-// range; what follows is not used then. weak: the row's entries that need a look (served).
-__device__ __forceinline__ bool factor_diagonal(int64_t* blk, int rows, int cols, Rsqrt* rsq, uint32_t& row, int l16,
+// range; what follows is not used then. weak: the row's weak entries (fix64.cuh).
+__device__ __forceinline__ bool factor_diagonal(int64_t* blk, int rows, int cols, Rsqrt* rsq, uint32_t& row, int J, int l16,
                                                 uint32_t below, unsigned& weak) {
     blk += l16;
-    int64_t acc[kB], cr[kB];
+    int64_t sum[kB], cross[kB];
 #pragma unroll
     for (int c = 0; c < kB; ++c) {
-        acc[c] = l16 < cols ? blk[c * kS] : 0;
-        cr[c] = -fix64::kCrossStart;
+        sum[c] = l16 < cols ? blk[c * kS] : 0;
+        cross[c] = fix64::kCrossOfRemainder;
     }
     bool good = true, off = false;
-    int64_t squares = 0;
+    int64_t squares = 0, t = 0;
     int any = 0;
+    Rsqrt y;
     // The next pivot's reciprocal square root is taken as soon as its column is up to date, beside the
     // products of the columns after it.
-    int64_t t = 0;
-    Rsqrt y;
     auto pivot = [&](int c) {
-        t = acc[c] - fix64::total(0, -cr[c]);
+        t = fix64::remainder_of(sum[0], cross[0]);
         int64_t const s = __shfl_sync(0xffffffffu, t, c, kB);
         good &= s >= fix64::kPivotMin || c >= rows;
         y = fix64::pivot_rsqrt(max(s, fix64::kPivotMin));
     };
     pivot(0);
-#pragma unroll
-    for (int j = 0; j < kB; ++j) {
-        if (j < cols) {
-            int64_t q;
-            bool const ok = fix64::scale_entry(t, y, q);
-            Limbs const v = fix64::split(q);
-            blk[j * kS] = fix64::pack(v);
-            if (fix64::weak(t, below)) weak |= 1u << j;
-            if (l16 >= j) {
-                off |= !ok;
-                fix64::add_square(squares, v.h);
-                any |= v.h | v.l;
-            }
-            if (l16 == 0) rsq[j] = y;
-            int const nh = -v.h, nl = -v.l;
-#pragma unroll
-            for (int c = j + 1; c < kB; ++c) {
-                int const h = __shfl_sync(0xffffffffu, v.h, c, kB), l = __shfl_sync(0xffffffffu, v.l, c, kB);
-                fix64::mad(acc[c], nh, h);
-                fix64::mad(cr[c], nh, l);
-                fix64::mad(cr[c], nl, h);
-                if (c == j + 1) pivot(c);
-            }
+    fix64::triangle(cols, [&](auto left, int j) {
+        int64_t q;
+        bool const ok = fix64::scale_entry(t, y, q);
+        Limbs const v = fix64::split(q);
+        blk[j * kS] = fix64::pack(v);
+        if (l16 >= j) {
+            off |= !ok;
+            fix64::add_square(squares, v.h);
         }
-    }
-    weak &= l16 < rows ? (1u << l16) - 1 : 0;
+        if (l16 > j) {
+            if (fix64::weak(t, below)) weak |= 1u << j;
+            any |= v.h | v.l;
+        }
+        if (l16 == 0) rsq[j] = y;
+#pragma unroll
+        for (int u = 1; u < decltype(left)::value; ++u) {
+            int const c = j + u;  // past the last column: sums that are not used
+            fix64::take_off(sum, cross, u, v, Limbs{__shfl_sync(0xffffffffu, v.l, c, kB), __shfl_sync(0xffffffffu, v.h, c, kB)});
+            if (u == 1) pivot(c);
+        }
+    });
     if (l16 >= rows) return good;
-    return add_row(row, squares, any) && good && !off;
+    row = fix64::row_after(row, J, squares, any != 0);
+    return (row & fix64::kNormMask) <= fix64::kNormMost && good && !off;
 }
 
 // A row (this lane's, at x) against the diagonal block D; mine: the row exists (else it becomes zeros). False if
 // it is out of range.
-__device__ __forceinline__ bool solve_block_row(int64_t* x_at, bool mine, const int64_t* D, const Rsqrt* rsq, uint32_t& row,
-                                                uint32_t below, unsigned& weak) {
-    Limbs x[kB];
+__device__ __forceinline__ bool solve_block_row(int64_t* x, bool mine, const int64_t* D, const Rsqrt* rsq, uint32_t& row,
+                                                int J, uint32_t below, unsigned& weak) {
+    int64_t sum[kB], cross[kB];
+#pragma unroll
+    for (int c = 0; c < kB; ++c) {
+        sum[c] = mine ? x[c * kS] : 0;
+        cross[c] = fix64::kCrossOfRemainder;
+    }
     bool ok = true;
     int64_t squares = 0;
     int any = 0;
-#pragma unroll
-    for (int j = 0; j < kB; ++j) {
-        int64_t hh = 0, c0 = fix64::kCrossStart, c1 = 0;
-#pragma unroll
-        for (int q = 0; q < j; ++q) {
-            Limbs const d = fix64::unpack(D[q * kS + j]);
-            fix64::mad(hh, x[q].h, d.h);
-            fix64::mad(c0, x[q].h, d.l);
-            fix64::mad(c1, x[q].l, d.h);
-        }
-        int64_t v;
-        int64_t const t = (mine ? x_at[j * kS] : 0) - fix64::total(hh, c0 + c1);
-        ok &= fix64::scale_entry(t, rsq[j], v);
+    fix64::triangle(kB, [&](auto left, int j) {
+        int64_t q;
+        int64_t const t = fix64::remainder_of(sum[0], cross[0]);
+        ok &= fix64::scale_entry(t, rsq[j], q);
         if (fix64::weak(t, below)) weak |= 1u << j;
-        x[j] = fix64::split(v);
-        x_at[j * kS] = fix64::pack(x[j]);
-        fix64::add_square(squares, x[j].h);
-        any |= x[j].h | x[j].l;
-    }
-    return add_row(row, squares, any) && ok;
+        Limbs const v = fix64::split(q);
+        x[j * kS] = fix64::pack(v);
+        fix64::add_square(squares, v.h);
+        any |= v.h | v.l;
+        int64_t const* d = D + j * (kS + 1);
+#pragma unroll
+        for (int u = 1; u < decltype(left)::value; ++u) fix64::take_off(sum, cross, u, v, fix64::unpack(d[u]));
+    });
+    row = fix64::row_after(row, J, squares, any != 0);
+    return (row & fix64::kNormMask) <= fix64::kNormMost && ok;
 }
 
-// Whether the weak entries of rows first + l16 (a lane's, those of n) in block column J are served by fixed point all
-// the same (fix64.cuh). row: the rows' words; A: the matrix. A row without any entry so far is its lane's affair; other
-// entries are looked at by their matrix's 16 lanes together, one entry of each matrix at a time.
-__device__ __forceinline__ bool served(const int64_t* P, const uint32_t* row, const double* A, int64_t lda, int n, int first,
-                                       int J, uint32_t below, unsigned weak, int l16) {
-    int const base = kB * J, shift = threadIdx.x & 16;
-    auto entry = [&](int r, int c) { return P[block_at(r / kB, c / kB) + c % kB * kS + r % kB]; };
-    auto half = [&](bool x) { return (__ballot_sync(0xffffffffu, x) >> shift) & 0xffffu; };
-    bool ok = true;
-    if (weak != 0 && (row[first + l16] & fix64::kSeen) == 0) {
-        for (; weak != 0; weak &= weak - 1) ok &= A[first + l16 + (base + __ffs(weak) - 1) * lda] == 0.0;
-    }
-    for (;;) {
-        unsigned const who = half(weak != 0);
-        if (!__any_sync(0xffffffffu, who != 0)) return ok;
-        int const src = max(__ffs(who) - 1, 0), i = first + src;
-        int const j = base + max(__ffs(__shfl_sync(0xffffffffu, weak, src, kB)) - 1, 0);
-        unsigned through = 0, terms = 0;
-        auto look = [&](int k) {
-            int64_t a = 0, b = 0;
-            if (who != 0 && k < n && k != i && k != j) a = entry(max(i, k), min(i, k)), b = entry(max(j, k), min(j, k));
-            through |= half(fix64::strong(fix64::unpack(a).h, fix64::unpack(b).h, below));
-            terms |= half(k < j && a != 0 && b != 0);
-        };
-        look(base + l16);
-        if (__any_sync(0xffffffffu, who != 0 && through == 0)) {
-            for (int K = 0; K < J; ++K) look(kB * K + l16);
-            // an entry of zero without terms is exact
-            if (l16 == src && who != 0 && through == 0 && (terms != 0 || entry(i, j) != 0 || A[i + j * lda] != 0.0)) ok = false;
+// Whether fixed point serves row i in block column J although some of its entries are weak (fix64.cuh); a lane's own
+// affair. row: the rows' words; A: the matrix, n rows. Out of line, and as few instructions as can be: they are not in the
+// instruction cache when they are wanted.
+__device__ __noinline__ bool served(const int64_t* P, const uint32_t* row, const double* A, int64_t lda, int n, int i, int J,
+                                    uint32_t below, unsigned weak) {
+    int const base = kB * J, end = min(n, base + kB), first = fix64::first_panel(row[i]);
+    auto entry = [&](int r, int c) { return fix64::unpack(P[block_at(r / kB, c / kB) + c % kB * kS + r % kB]); };
+    unsigned zeros = 0;
+    for (; weak != 0 && first <= J; weak &= weak - 1) {
+        int const j = base + __ffs(weak) - 1;
+        uint32_t terms = 0;
+        bool any = false;
+#pragma unroll 1
+        for (int k = kB * min(J, max(first, fix64::first_panel(row[j]))); k < end && terms < below; ++k) {
+            if (k == i || k == j) continue;
+            Limbs const a = entry(max(i, k), min(i, k)), b = entry(max(j, k), min(j, k));
+            terms += fix64::term(a.h, b.h);
+            any |= k < j && (a.h | a.l) != 0 && (b.h | b.l) != 0;
         }
-        if (l16 == src) weak = ok ? weak & (weak - 1) : 0;
+        if (terms < below) {
+            Limbs const q = entry(i, j);
+            if (any || (q.h | q.l) != 0) return false;
+            zeros |= 1u << (j - base);
+        }
     }
+    if ((zeros | weak) == 0) return true;
+    bool exact = true;
+#pragma unroll 4
+    for (int j = 0; j < kB; ++j)
+        if (((zeros | weak) >> j & 1) != 0) exact &= A[i + (base + j) * lda] == 0.0;
+    return exact;
 }
 
 // 1 / d, the same bits for d times a power of two.
@@ -455,7 +443,7 @@ __global__ void __launch_bounds__(32, 8) posv_pair_kernel(Batch batch, int64_t c
         int e = 0;
         if (i < n) sound &= fix64::scale_exponent(__longlong_as_double(P[block_at(i / kB, i / kB) + i % kB * (kS + 1)]), e);
         scale[i] = e;
-        row[i] = 0;
+        row[i] = fix64::kNewRow;
     }
     unsigned const half_mask = 0xffffu << (16 * half);
     uint32_t const below = fix64::weak_below(n);
@@ -471,16 +459,17 @@ __global__ void __launch_bounds__(32, 8) posv_pair_kernel(Batch batch, int64_t c
         __syncwarp();
         auto look = [&](int first, unsigned weak) {
             __syncwarp();
-            if (first + l16 >= n || redo != blocks) weak = 0;
-            if (__any_sync(0xffffffffu, weak != 0)) sound &= served(P, row, it.A, it.lda, n, first, J, below, weak, l16);
+            if (weak != 0 && first + l16 < n && sound && redo == blocks)
+                sound = served(P, row, it.A, it.lda, n, first + l16, J, below, weak);
         };
         unsigned weak = 0;
-        sound &= factor_diagonal(P + block_at(J, J), n - kB * J, min(kB, nmax - kB * J), rsq, row[kB * J + l16], l16, below, weak);
+        sound &= factor_diagonal(P + block_at(J, J), min(kB, n - kB * J), min(kB, nmax - kB * J), rsq, row[kB * J + l16], J, l16,
+                                 below, weak);
         look(kB * J, weak);
         for (int I = J + 1; I < blocks; ++I) {
             weak = 0;
             sound &= solve_block_row(P + block_at(I, J) + l16, kB * I + l16 < nmax, P + block_at(J, J), rsq, row[kB * I + l16],
-                                     below, weak);
+                                     J, below, weak);
             look(kB * I, weak);
         }
         __syncwarp();
@@ -493,20 +482,21 @@ __global__ void __launch_bounds__(32, 8) posv_pair_kernel(Batch batch, int64_t c
     if (SOLVE || !HOST || __any_sync(0xffffffffu, n > 0 && redo < blocks)) {
         for (int I = 0; I < blocks; ++I) {
             int const r = kB * I + l16, e = scale[r] - 61;
-            for (int J = 0; J <= I; ++J) {
+            for (int J = 0; J <= min(I, redo - 1); ++J) {
                 int64_t* blk = P + block_at(I, J) + l16;
                 double* l = it.L + r + (int64_t)(kB * J) * it.ldl;
-                double const* a = it.A + r + (int64_t)(kB * J) * it.lda;
-                bool const again = J >= redo;
 #pragma unroll 4
                 for (int c = 0; c < kB; ++c) {
-                    if (kB * J + c > r) continue;
-                    double x = 0.0;
-                    if (r < n) x = again ? a[c * it.lda] : fix64::entry_to_double(fix64::join(fix64::unpack(blk[c * kS])), e);
-                    if (SOLVE || redo < blocks) blk[c * kS] = __double_as_longlong(x);
-                    if (!HOST && !again && r < n) l[c * it.ldl] = x;
+                    bool const in = kB * J + c <= r;
+                    double const x = fix64::entry_to_double(fix64::join(fix64::unpack(blk[c * kS])), e);
+                    if (SOLVE || redo < blocks) blk[c * kS] = in && r < n ? __double_as_longlong(x) : 0;
+                    if (!HOST && in && r < n) l[c * it.ldl] = x;
                 }
             }
+            for (int J = redo; J <= I; ++J)
+                for (int c = 0; c < kB; ++c)
+                    P[block_at(I, J) + l16 + c * kS] =
+                        kB * J + c <= r && r < n ? __double_as_longlong(it.A[r + (int64_t)(kB * J + c) * it.lda]) : 0;
         }
         if (redo < blocks && n > 0) {
             double* F = reinterpret_cast<double*>(P);
@@ -560,17 +550,13 @@ struct PairDesc {
     }
 };
 
-constexpr size_t kFourPerSm = 48 * 1024;
-
 template <bool SOLVE, bool HOST = false, class Batch>
 int launch(Batch const& batch, int max_n, int64_t count, int32_t* info, cudaStream_t s) {
     if (count == 0) return BLASTGPU_SUCCESS;
     if (max_n > kMaxN || (count + 1) / 2 > 0x7fffffff) return BLASTGPU_ERR_TOO_LARGE;
     int const N = (max_n + kB - 1) / kB;
-    // At N = 4 a fifth warp fits an SM, which helps the solves (n = 64 x 20,000: 3.0 ms, 3.4 with four) and leaves the
-    // schedulers uneven for the factor alone (n = 60 x 20,000: 1.49 ms, 1.33 with four).
-    size_t const smem = SOLVE || N < 4 ? 2 * (size_t)layout_of(N).bytes : kFourPerSm;
-    cudaError_t const e = ensure_smem<posv_pair_kernel<SOLVE, HOST, Batch>>(kFourPerSm);
+    size_t const smem = 2 * (size_t)layout_of(N).bytes;
+    cudaError_t const e = ensure_smem<posv_pair_kernel<SOLVE, HOST, Batch>>(2 * (size_t)layout_of(kMaxN / kB).bytes);
     if (e != cudaSuccess) { set_cuda_error(e); return BLASTGPU_ERR_CUDA; }
     posv_pair_kernel<SOLVE, HOST, Batch><<<(unsigned)((count + 1) / 2), 32, smem, s>>>(batch, count, N, info);
     return check_launch();

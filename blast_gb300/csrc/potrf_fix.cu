@@ -329,96 +329,92 @@ __device__ __forceinline__ int64_t from_workspace(int64_t w) {
 // Why the panels end early: a row, or the whole panel, is left to binary64.
 constexpr int kStopRow = 1, kStopPanel = 2;
 
+// A panel from the side of its rows: entry (i, j) is in row k0 + i and column k0 + j.
 struct Panel {
     int k0, nb;
-    const double* A;
+    const double* A;  // the matrix from (0, 0) of the panel on
     int64_t lda;
-    int64_t* W;
+    int64_t* W;       // the workspace's columns from row k0 on
     int64_t ldw;
-    const Limbs* D;  // the diagonal block, row by row
-    uint32_t* row;   // the rows' words
-    uint32_t below;  // fix64::weak_below
+    const Limbs* D;   // the diagonal block, row by row
+    uint32_t* row;    // the rows' words
+    uint32_t below;   // fix64::weak_below
     int* stop;
 };
 
-// Whether the weak entries of the warp's rows first + lane of the panel are served by fixed point all the same
-// (fix64.cuh). C: the chunk's columns at row `first`, with the entries of the rows that have weak ones. The warp
-// looks at one entry at a time.
+// Whether fixed point serves row i although some of its entries in the panel are weak (fix64.cuh). x: those entries,
+// CS apart; one thread.
 template <int T>
-__device__ __noinline__ bool served(int first, int nb, int k0, const int64_t* C, const Limbs* D, const int64_t* W, int64_t ldw,
-                                    const double* A, int64_t lda, const uint32_t* words, uint32_t below, unsigned weak) {
+__device__ __forceinline__ bool served(Panel const& p, int i, const int64_t* x, unsigned weak) {
     using S = Shape<T>;
-    int const lane = threadIdx.x & 31;
-    bool ok = true;
-    for (;;) {
-        unsigned const who = __ballot_sync(0xffffffffu, weak != 0);
-        if (who == 0) return ok;
-        int const src = __ffs(who) - 1, i = first + src, j = __ffs(__shfl_sync(0xffffffffu, weak, src)) - 1;
-        bool through = false, term = false;
-        if (lane < nb && lane != i && lane != j) {
-            int const k = lane;
-            Limbs const u = k < i ? fix64::split(C[k * S::CS + src]) : D[k * kNB + i];
-            Limbs const v = D[max(j, k) * kNB + min(j, k)];
-            through = fix64::strong(u.h, v.h, below);
-            term = k < j && (u.h | u.l) != 0 && (v.h | v.l) != 0;
-        }
-        int const before = (words[i] & words[j] & fix64::kSeen) ? k0 : 0;
-        for (int k = lane; !__any_sync(0xffffffffu, through) && k - lane < before; k += 32) {
-            if (k < before) {
-                int64_t const u = from_workspace<T>(W[i + k * ldw]), v = from_workspace<T>(W[j + k * ldw]);
-                through = fix64::strong(fix64::high_limb(u), fix64::high_limb(v), below);
-                term |= u != 0 && v != 0;
+    int const J = p.k0 / kNB, first = fix64::first_panel(p.row[i]);
+    unsigned zeros = 0;
+    for (; weak != 0 && first <= J; weak &= weak - 1) {
+        int const j = __ffs(weak) - 1;
+        uint32_t terms = 0;
+        bool any = false;
+#pragma unroll 1
+        for (int k = kNB * max(first, fix64::first_panel(p.row[j])); k < p.k0 && terms < p.below; k += 2) {
+            int64_t u[2], v[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) u[c] = p.W[i + (k + c) * p.ldw], v[c] = p.W[j + (k + c) * p.ldw];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                int64_t const a = from_workspace<T>(u[c]), b = from_workspace<T>(v[c]);
+                terms += fix64::term(fix64::split(a).h, fix64::split(b).h);
+                any |= a != 0 && b != 0;
             }
         }
-        // an entry of zero without terms is exact
-        bool const fine = __any_sync(0xffffffffu, through) ||
-                          !(__any_sync(0xffffffffu, term) || C[j * S::CS + src] != 0 || A[i + j * lda] != 0.0);
-        if (lane == src) {
-            ok = fine;
-            weak = ok ? weak & (weak - 1) : 0;
+#pragma unroll 1
+        for (int k = 0; k < p.nb && terms < p.below; ++k) {
+            if (k == i || k == j) continue;
+            Limbs const a = k < i ? fix64::split(x[k * S::CS]) : p.D[k * kNB + i];
+            Limbs const b = p.D[max(j, k) * kNB + min(j, k)];
+            terms += fix64::term(a.h, b.h);
+            any |= k < j && (a.h | a.l) != 0 && (b.h | b.l) != 0;
+        }
+        if (terms < p.below) {
+            if (any || x[j * S::CS] != 0) return false;
+            zeros |= 1u << j;
         }
     }
+    if ((zeros | weak) == 0) return true;
+    bool exact = true;
+#pragma unroll 4
+    for (int j = 0; j < kNB; ++j)
+        if (((zeros | weak) >> j & 1) != 0) exact &= p.A[i + j * p.lda] == 0.0;
+    return exact;
 }
 
-// Whether the warp's rows first + lane of the panel (mine: the lane has one) are certified; their words after the
-// panel. C: the chunk's columns at row `first`; q: the row's entries.
+// What a row's way through the panel leaves.
+struct RowState {
+    bool ok = true;  // in range
+    unsigned weak = 0;  // entries
+    int64_t squares = 0;
+    int any = 0;
+};
+
+// Whether row i is certified; its word after the panel. One thread. Out of line, and as few instructions as can be:
+// what is executed once in a while is not in the instruction cache (n = 128 x 4,000, with five weak entries a
+// matrix: 1.72 ms, 2.05 when a row with one was gone through entry by entry, 1.51 without a look at them).
 template <int T>
-__device__ __forceinline__ bool certify(Panel const& p, int first, bool mine, const int64_t (&q)[kNB], int64_t* C, bool ok,
-                                        unsigned weak, int64_t squares, int any) {
-    int const lane = threadIdx.x & 31;
-    if (mine) {
-        uint32_t* const word = p.row + p.k0 + first + lane;
-        uint32_t const w = *word, now = (w + fix64::norm_of(squares)) | (any != 0 ? fix64::kSeen : 0);
-        ok &= (w & fix64::kTodo) == 0 && (now & fix64::kNormMask) <= fix64::kNormMost;
-        *word = now;
-        if ((now & fix64::kSeen) == 0)  // a row without any entry so far
-            for (; weak != 0; weak &= weak - 1)
-                ok &= p.A[p.k0 + first + lane + (p.k0 + __ffs(weak) - 1) * p.lda] == 0.0;
-    }
-    if (!mine || !ok) weak = 0;
-    if (__any_sync(0xffffffffu, weak != 0)) {
-        if (weak != 0) {
-#pragma unroll
-            for (int j = 0; j < kNB; ++j) C[j * Shape<T>::CS + lane] = q[j];
-        }
-        __syncwarp();
-        ok &= served<T>(first, p.nb, p.k0, C, p.D, p.W + p.k0, p.ldw, p.A + p.k0 + p.k0 * p.lda, p.lda, p.row + p.k0, p.below, weak);
-    }
-    return ok;
+__device__ __noinline__ bool certified(Panel const p, int i, const int64_t* x, RowState const s) {
+    uint32_t const now = fix64::row_after(p.row[i], p.k0 / kNB, s.squares, s.any != 0);
+    p.row[i] = now;
+    return s.ok && (now & fix64::kTodo) == 0 && (now & fix64::kNormMask) <= fix64::kNormMost &&
+           (s.weak == 0 || served<T>(p, i, x, s.weak));
 }
 
-// A row that was taken through the panel: stored if it is certified, else left to binary64.
+// Row i of the panel to the workspace, its first `entries` columns, if it is certified; else it is left to binary64.
 template <int T>
-__device__ __forceinline__ void finish_row(Panel const& p, int i, int entries, const int64_t (&q)[kNB], bool ok) {
-    if (ok) {
-        int64_t* w = p.W + p.k0 + i + p.k0 * p.ldw;
-#pragma unroll
-        for (int j = 0; j < kNB; ++j)
-            if (j < entries) w[j * p.ldw] = to_workspace<T>(q[j]);
-    } else {
-        p.row[p.k0 + i] |= fix64::kTodo;
+__device__ __forceinline__ void store_row(Panel const& p, int i, int entries, const int64_t* x, bool ok) {
+    if (!ok) {
+        p.row[i] |= fix64::kTodo;
         *p.stop = kStopRow;
+        return;
     }
+#pragma unroll 4
+    for (int j = 0; j < entries; ++j) p.W[i + (p.k0 + j) * p.ldw] = to_workspace<T>(x[j * Shape<T>::CS]);
 }
 
 // The panel's first 32 rows (mr of them exist), one warp, a row per lane: the 16 columns right-looking.
@@ -428,97 +424,82 @@ __device__ __forceinline__ void factor_diagonal(Panel const& p, int mr, int64_t*
     using S = Shape<T>;
     int const lane = threadIdx.x & 31, nb = p.nb;
     bool const mine = lane < mr;
-    int64_t acc[kNB], cr[kNB];  // acc: column j's entry q once it is there
+    int64_t sum[kNB], cross[kNB];
 #pragma unroll
     for (int c = 0; c < kNB; ++c) {
-        acc[c] = mine && c < nb ? C[c * S::CS + lane] : 0;
-        cr[c] = fix64::kCrossStart;
+        sum[c] = mine && c < nb ? C[c * S::CS + lane] : 0;
+        cross[c] = fix64::kCrossOfRemainder;
     }
-    bool good = true, ok = true;
-    unsigned weak = 0;
-    int64_t squares = 0;
-    int any = 0;
+    bool good = true;
+    RowState state;
     // The next pivot's reciprocal square root is taken as soon as its column is up to date, beside the
     // products of the columns after it.
     int64_t t = 0;
     Rsqrt y;
     auto pivot = [&](int c) {
-        t = acc[c] - fix64::total(0, cr[c]);
+        t = fix64::remainder_of(sum[0], cross[0]);
         int64_t const s = __shfl_sync(0xffffffffu, t, c);
-        good &= s >= fix64::kPivotMin;
+        good &= s >= fix64::kPivotMin || c >= nb;
         y = fix64::pivot_rsqrt(max(s, fix64::kPivotMin));
     };
     pivot(0);
-#pragma unroll
-    for (int j = 0; j < kNB; ++j) {
-        if (j < nb) {  // warp-uniform
-            int64_t q;
-            bool const in = fix64::scale_entry(t, y, q);
-            Limbs const v = fix64::split(q);
-            acc[j] = q;
-            if (fix64::weak(t, p.below)) weak |= 1u << j;
-            if (lane >= j) {
-                ok &= in;
-                fix64::add_square(squares, v.h);
-                any |= v.h | v.l;
-            }
-            if (lane < kNB) D[lane * kNB + j] = v;
-            if (lane == 0) rsq[j] = y;
-#pragma unroll
-            for (int c = j + 1; c < kNB; ++c) {
-                int const h = __shfl_sync(0xffffffffu, v.h, c), l = __shfl_sync(0xffffffffu, v.l, c);
-                fix64::mad(acc[c], -v.h, h);
-                fix64::mad(cr[c], v.h, l);
-                fix64::mad(cr[c], v.l, h);
-                if (c == j + 1 && c < nb) pivot(c);
-            }
+    fix64::triangle(nb, [&](auto left, int j) {
+        int64_t q;
+        bool const in = fix64::scale_entry(t, y, q);
+        Limbs const v = fix64::split(q);
+        if (lane >= j) {
+            state.ok &= in;
+            fix64::add_square(state.squares, v.h);
         }
-    }
-    weak &= lane < kNB ? (1u << lane) - 1 : 0xffffu;
+        if (lane > j) {
+            if (fix64::weak(t, p.below)) state.weak |= 1u << j;
+            state.any |= v.h | v.l;
+        }
+        if (mine) C[j * S::CS + lane] = q;
+        if (lane < kNB) D[lane * kNB + j] = v;
+        if (lane == 0) rsq[j] = y;
+#pragma unroll
+        for (int u = 1; u < decltype(left)::value; ++u) {
+            int const c = j + u;  // past the last column: sums that are not used
+            fix64::take_off(sum, cross, u, v, Limbs{__shfl_sync(0xffffffffu, v.l, c), __shfl_sync(0xffffffffu, v.h, c)});
+            if (u == 1) pivot(c);
+        }
+    });
     __syncwarp();
     // The diagonal block's rows are certified before any row is stored.
-    ok = certify<T>(p, 0, mine, acc, C, ok, weak, squares, any);
-    if (__all_sync(0xffffffffu, good && (ok || lane >= nb || !mine))) {
-        if (mine) finish_row<T>(p, lane, min(lane + 1, kNB), acc, ok);
+    bool const ok = mine && certified<T>(p, lane, C + lane, state);
+    if (__all_sync(0xffffffffu, good && (ok || !mine || lane >= nb))) {
+        if (mine) store_row<T>(p, lane, min(lane + 1, nb), C + lane, ok);
     } else if (lane == 0) {
         *p.stop = kStopPanel;
     }
 }
 
-// A warp's rows first + lane of the panel, r = r0 + lane of the chunk (mine: the lane has one), against the diagonal
-// block.
+// Row i of the panel, r of the chunk, against the diagonal block, one thread.
 template <int T>
-__device__ __forceinline__ void solve_rows(Panel const& p, int first, int r0, bool mine, int64_t* C, const Limbs* D,
-                                           const Rsqrt* rsq) {
+__device__ __forceinline__ void solve_row(Panel const& p, int i, int r, int64_t* C, const Limbs* D, const Rsqrt* rsq) {
     using S = Shape<T>;
-    int const r = r0 + (threadIdx.x & 31);
-    Limbs x[kNB];
-    int64_t v[kNB];
-    bool ok = true;
-    unsigned weak = 0;
-    int64_t squares = 0;
-    int any = 0;
+    int64_t sum[kNB], cross[kNB];
 #pragma unroll
-    for (int j = 0; j < kNB; ++j) {
-        int64_t hh = 0, c0 = fix64::kCrossStart, c1 = 0;
-#pragma unroll
-        for (int q = 0; q < j; ++q) {
-            Limbs const d = D[j * kNB + q];
-            fix64::mad(hh, x[q].h, d.h);
-            fix64::mad(c0, x[q].h, d.l);
-            fix64::mad(c1, x[q].l, d.h);
-        }
-        int64_t const t = C[j * S::CS + r] - fix64::total(hh, c0 + c1);
-        ok &= fix64::scale_entry(t, rsq[j], v[j]);
-        if (fix64::weak(t, p.below)) weak |= 1u << j;
-        x[j] = fix64::split(v[j]);
-        fix64::add_square(squares, x[j].h);
-        any |= x[j].h | x[j].l;
+    for (int c = 0; c < kNB; ++c) {
+        sum[c] = C[c * S::CS + r];
+        cross[c] = fix64::kCrossOfRemainder;
     }
+    RowState state;
+    fix64::triangle(kNB, [&](auto left, int j) {
+        int64_t q;
+        int64_t const t = fix64::remainder_of(sum[0], cross[0]);
+        state.ok &= fix64::scale_entry(t, rsq[j], q);
+        if (fix64::weak(t, p.below)) state.weak |= 1u << j;
+        Limbs const v = fix64::split(q);
+        C[j * S::CS + r] = q;
+        fix64::add_square(state.squares, v.h);
+        state.any |= v.h | v.l;
+        Limbs const* d = D + j * (kNB + 1);  // past the last row: what follows D, for sums that are not used
 #pragma unroll
-    for (int j = 0; j < kNB; ++j) v[j] = fix64::join(x[j]);
-    ok = certify<T>(p, first, mine, v, C + r0, ok, weak, squares, any);
-    if (mine) finish_row<T>(p, first + (threadIdx.x & 31), kNB, v, ok);
+        for (int u = 1; u < decltype(left)::value; ++u) fix64::take_off(sum, cross, u, v, d[u * kNB]);
+    });
+    store_row<T>(p, i, kNB, C + r, certified<T>(p, i, C + r, state));
 }
 
 // One matrix. W: the fixed-point factor while the matrix is being factored, n rows of 8 bytes per
@@ -558,14 +539,14 @@ __global__ void __launch_bounds__(T, T == 128 ? 3 : T == 64 ? 7 : 11) potrf_fix_
         int e;
         if (!fix64::scale_exponent(it.A[i + (int64_t)i * it.lda], e)) s_stop = kStopPanel;
         scale[i] = (short)e;
-        row[i] = 0;
+        row[i] = fix64::kNewRow;
     }
     cta_sync<T>();
     uint32_t const below = fix64::weak_below(n);
     int stop = s_stop, k0 = 0, r0 = 0;
     for (; k0 < n && stop == 0; k0 += stop == 0 ? kNB : 0) {
         int const nb = min(kNB, n - k0), m = n - k0;
-        Panel const p{k0, nb, it.A, it.lda, W, it.ldw, D, row, below, &s_stop};
+        Panel const p{k0, nb, it.A + k0 + k0 * it.lda, it.lda, W + k0, it.ldw, D, row + k0, below, &s_stop};
         for (r0 = 0; r0 < m && stop == 0; r0 += stop == 0 ? T : 0) {
             int const mr = min(T, m - r0);
             if constexpr (S::kTensor) {
@@ -587,9 +568,7 @@ __global__ void __launch_bounds__(T, T == 128 ? 3 : T == 64 ? 7 : 11) potrf_fix_
                 cta_sync<T>();
             }
             // Nobody writes kStopPanel from here on, so every thread sees the same side of it.
-            int const warp_row = tid & ~31;
-            if (s_stop != kStopPanel && warp_row < mr && (r0 > 0 || warp_row > 0))
-                solve_rows<T>(p, r0 + warp_row, warp_row, tid < mr, C, D, rsq);
+            if (s_stop != kStopPanel && tid < mr && (r0 > 0 || tid >= 32)) solve_row<T>(p, r0 + tid, tid, C, D, rsq);
             cta_sync<T>();  // C is written again; the panel's columns are read from now on
             stop = s_stop;  // not written again before the next chunk's barriers
         }
