@@ -684,17 +684,44 @@ bool posv_quad_wanted(PosvArgs const& p) {
     return p.batch * 100 < (int64_t)t * 32 * 4 * sms;
 }
 
-// Whether a uniform batch is factored in fixed point. That cost goes by the size rounded up to 16, and a
-// warp's worth of matrices needs few warps; the thread-per-matrix kernel's goes by the size, and it needs a
-// batch that gives every scheduler two full warps. Measured on GB300 (binary64 against fixed point, us, 8
-// right-hand sides): n = 17 x 3,000: 92, 59; x 50,000: 537, 813. n = 20 x 10,000: 186, 171, the factor alone 78, 85.
-// n = 24 x 50,000: 963, 931, the factor alone 371, 415. n = 33 x 10,000: 534, 515; x 50,000: 1,954, 2,391. n = 40 x
-// 50,000: 2,689, 2,649. n = 52 x 50,000: 4,957, 5,530. Above 64 the fixed-point factor has a CTA to a matrix: n = 65
-// x 3,000: 1,370, 1,127; x 6,000: 1,556, 1,678; n = 76 x 10,000: 2,938, 2,746.
-bool fixed_point_wanted(int n, int64_t batch) {
+// Whether a uniform batch is factored in fixed point, and up to n = 64 solved by the pair kernel. Their cost
+// goes by the size rounded up to 16 and starts from few matrices; the thread-per-matrix kernel's goes by the size, by 8
+// right-hand sides at a time, and it needs a batch that gives every scheduler full warps (quads help below
+// 1.5). So the share of the rounded size that is used decides, against the full warps of matrices per
+// scheduler. Measured on GB300 (binary64 / fixed point, us; 19,456 matrices are one warp per scheduler), right-hand sides
+// none, 1 and 8:
+//   n = 17 x 3,000: 43/36, 78/51, 93/87; x 10,000: 75/87, 136/140, 167/274
+//   n = 21 x 20,000: 215/183, 384/269, 469/579; x 50,000: 298/430, 723/601, 804/1351
+//   n = 28 x 20,000: 317/228, 557/306, 692/624; x 50,000: 535/539, 1179/690, 1323/1460
+//   n = 40 x 20,000: 702/512, 1122/692, 1439/1367; x 50,000: 1278/1203, 2548/1628, 2697/3213
+//   n = 48 x 50,000: 2133/1407, 3934/1839, 4148/3419; n = 53 x 20,000: 1598/1178, 2356/1539, 2855/2676
+// Above 64 the factor has a CTA to a matrix, whatever the right-hand sides: n = 68 x 3,000: 726/440, x 10,000: 1337/1489;
+// n = 72 x 10,000: 1558/1525, n = 80 2083/1587.
+// In host memory the link is what counts, and the thread kernel leaves it idle unless the batch fills the chip: n = 24 x
+// 10,000, one batch at a time 806/570, three in flight 446/430; x 50,000: 2177/2208, 1681/2056; n = 40 x 30,000: 3212/3199,
+// 2365/2813; n = 60 x 30,000: 6925/5334, 5066/5011.
+bool fixed_point_wanted(int n, int nrhs, int64_t batch, bool host) {
     if (n < kFixMinN || n > 512) return false;
-    if (batch >= 40000 && (n < 25 || (n <= 64 && (n & 15) >= 1 && (n & 15) <= 5))) return false;
-    return batch < 5000 || (n > 20 && (n <= 64 || n > 72));
+    double const warps = (double)batch / (32.0 * 4 * sm_count());
+    if (n > kPairMaxN) return n >= 72 || warps < 0.2 + 0.02 * (n - 64);
+    if (warps < (host ? 1.0 : 0.2)) return true;
+    int const used = 100 * n / (16 * ((n + 15) / 16));
+    if (host) return used >= 90;
+    bool const full = warps >= 1.5;
+    if (nrhs == 0) return used >= (full ? 80 : 64);
+    if (nrhs <= 2) return used >= 62;
+    if (nrhs <= 4) return used >= (full ? 80 : 70);
+    return used >= (full || nrhs > 8 ? 90 : 82);
+}
+
+// Whether solves with given factors run a CTA per matrix, a right-hand side at a time, instead of a thread or a quad
+// of lanes. "posv.cta_min_n" (default 65): from this n on. A CTA's time goes by batch and right-hand sides, a thread's by
+// groups of 8 right-hand sides, and hardly by the batch until it fills the chip. Measured on GB300 (CTA, thread, us): n = 65, one right-hand side x 100: 38, 312; x 2,000:
+// 220, 352; x 4,000: 459, 388; 8 right-hand sides x 100: 243, 478; x 1,000: 945, 484. n = 128, 8 x 1,000: 1,458, 1,609; x 2,000:
+// 2,579, 1,942; 16 x 700: 2,167, 3,092; 1 x 20,000: 3,414, 3,743. n = 256, 8 x 2,000: 6,112, 7,774; x 4,000: 12,013, 8,450.
+bool potrs_cta_wanted(int n, int nrhs, int64_t batch) {
+    if (n < tune_get("posv.cta_min_n", 65) || n > 512) return false;
+    return (double)batch * nrhs * 152 < 100.0 * (n - 25) * ((nrhs + 7) / 8) * sm_count();
 }
 
 int launch_posv(PosvArgs const& p, cudaStream_t stream) {
@@ -705,7 +732,8 @@ int launch_posv(PosvArgs const& p, cudaStream_t stream) {
         }
         return BLASTGPU_SUCCESS;
     }
-    if ((p.m == 0 || p.m == p.n) && p.mode != 2 && fixed_point_wanted(p.n, p.batch)) {
+    if ((p.m == 0 || p.m == p.n) && p.mode != 2 &&
+        fixed_point_wanted(p.n, p.mode == 1 ? p.nrhs : 0, p.batch, false)) {
         if (p.n <= kPairMaxN)
             return launch_posv_pair(p.n, p.mode == 1 ? p.nrhs : 0, p.A, p.lda, p.sa, p.L, p.ldl, p.sl, p.B, p.ldb, p.sb,
                                     p.X, p.ldx, p.sx, p.info, p.batch, false, stream);
@@ -716,9 +744,7 @@ int launch_posv(PosvArgs const& p, cudaStream_t stream) {
         q.mode = 2;
         return launch_posv(q, stream);
     }
-    // Solves from "posv.cta_min_n" (default 65) on go to the CTA-per-matrix kernel: a batch of one
-    // thread per matrix leaves most of the chip idle.
-    if (p.mode == 2 && p.n >= tune_get("posv.cta_min_n", 65) && p.n <= 512)
+    if (p.mode == 2 && potrs_cta_wanted(p.n, p.nrhs, p.batch))
         return launch_potrs_cta_strided(p.n, p.nrhs, p.L, p.ldl, p.sl, p.B, p.ldb, p.sb, p.X, p.ldx, p.sx, p.batch,
                                         stream);
     // "posv.variant": CTA size and the occupancy the register allocation is bounded for (4: as 3,
@@ -865,7 +891,7 @@ int blastgpu_dposv_mirror_strided(int n, int nrhs, const double* A, int lda, int
     PosvArgs const p{n, nrhs, A, lda, stride_a, L_work, n, (int64_t)n * n, B, ldb, stride_b, X_work, n,
                      (int64_t)n * nrhs, info, batch, 1};
     MirrorOut const o{L, ldl, stride_l, X, ldx, stride_x};
-    if (!fixed_point_wanted(n, batch)) {
+    if (!fixed_point_wanted(n, nrhs, batch, true)) {
         posv_mirror_kernel<true><<<(unsigned)blocks, 32, 0, s>>>(p, o);
         return check_launch();
     }

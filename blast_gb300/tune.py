@@ -14,8 +14,8 @@ Tunable choices (read by the library through blastgpu_tune_set / tune_get_bin):
 * ``posv.mixed.n<bin>`` — ragged mixed-precision Cholesky factorisation per size bin (the modes of
   posv_cta_mixed_kernel); timed on the mixed workload's matrices (cond 1e2, 1e4, 1e6) and kept only
   if every instance converges.
-* ``posv.cta_min_n`` — uniform solves with a given factor from this n on run one CTA per matrix
-  instead of one thread per matrix.
+* ``posv.cta_min_n`` — uniform solves with a given factor may run one CTA per matrix from this n on (not timed by
+  this module: from 65 on the library weighs batch and right-hand sides).
 * ``posv.warp.n<bin>`` — ragged binary64 Cholesky solves with every n <= 128: the substitutions (and
   for n <= 16 the factor) by one warp (1) or one CTA (0) per matrix (within 10 n eps of each other).
 * ``posv.quad.n<bin>`` — uniform Cholesky batches that run in binary64 on a thread per matrix run a
@@ -209,33 +209,6 @@ def tune_posv_mixed(bins=(64, 128, 256, 512), count: int = 1536, modes=(0, 1, 2,
     return out
 
 
-def tune_posv_cta_min_n(ns=(48, 56, 64, 72, 80, 96, 112, 128), nrhs=8, batch=20_000) -> dict:
-    """The smallest n from which a uniform Cholesky solve stays faster one CTA per matrix."""
-    from .blast import col_major, posv
-
-    best = None
-    for n in ns:
-        A = col_major((batch,), n, n, "cuda")
-        G = torch.randn(batch, n, n, device="cuda", dtype=torch.float64)
-        A.copy_(G @ G.mT + n * torch.eye(n, device="cuda", dtype=torch.float64))
-        del G
-        B = col_major((batch,), n, nrhs, "cuda")
-        B.copy_(torch.randn(batch, n, nrhs, device="cuda", dtype=torch.float64))
-        L, X = col_major((batch,), n, n, "cuda"), col_major((batch,), n, nrhs, "cuda")
-        _lib.tune_set("posv.cta_min_n", 1 << 20)
-        t_thread = _time(lambda: posv(A, L, B, X), reps=5)
-        _lib.tune_set("posv.cta_min_n", n)
-        t_cta = _time(lambda: posv(A, L, B, X), reps=5)
-        del A, B, L, X
-        if t_cta < t_thread:
-            best = n if best is None else best
-        else:
-            best = None  # the CTA kernels must stay ahead from the chosen n on
-    value = best if best is not None else ns[-1] + 1
-    _lib.tune_set("posv.cta_min_n", value)
-    return {"posv.cta_min_n": int(value)}
-
-
 def tune_posv_warp(bins=(32, 64, 128), count: int = 4096) -> dict:
     """Ragged binary64 Cholesky solves per size bin (n <= 128): one warp (1) or one CTA (0) per
     matrix, on SPD matrices with n uniform in the bin and one right-hand side."""
@@ -270,7 +243,6 @@ def run(save: bool = True) -> dict:
     choices.update(tune_gemm())
     choices.update(tune_getrf())
     choices.update(tune_posv_mixed())
-    choices.update(tune_posv_cta_min_n())
     choices.update(tune_posv_warp())
     if save:
         CACHE_DIR.mkdir(parents=True, exist_ok=True)

@@ -222,10 +222,10 @@ int blastgpu_dtrmm_strided(int side, int uplo, int unit, int m, int n, double al
 /* ---------------------------------------------------------------------------------------------
  * potrf: lower Cholesky factor L of a symmetric positive definite n x n A (only the lower
  * triangle of A is read; the strict upper triangle of L is not written). L may equal A. Uniform
- * batches with n >= posv.cta_min_n (a tuning key: 65 unless set; the GB300 tuning cache that the
- * Python package applies sets 129) run one CTA per matrix in panels of 32 columns
- * (the ragged kernels' factorisation), below that one thread per matrix with BLAST's tiles; both
- * are within 10*n*eps of BLAST's algorithm. The same holds for posv and potrs below.
+ * batches run on binary64 threads (BLAST's tiles), two matrices per warp in fixed point (n <= 64) or a CTA per
+ * matrix in fixed point, by size, batch and right-hand sides; solves with a given factor on threads or, from
+ * n = posv.cta_min_n on (a tuning key: 65 unless set), also on a CTA per matrix. All are within
+ * 10*n*eps of BLAST's algorithm. The same holds for posv and potrs below.
  * Replaces blast::potrf(A, L) dense (dense/Potrf.hpp:66-106) and panel (panel/Potrf.hpp:59-106).
  * info[b] = 0, or j+1 if the j-th pivot was not positive (BLAST does not check and returns NaNs;
  * the factor is computed the same way and carries the same NaNs). info may be NULL.
