@@ -13,7 +13,7 @@ with the oracle (BLAST's algorithm restated in C++) and with LAPACK on a strided
 Prints one JSON line. `value` is matrices/s measured with CUDA events on the launching stream
 (max over ranks); `e2e` is the same metric through the public API with pinned host buffers and
 the host<->device traffic inside the timed region; `roofline` sets it against the binary64 FMA peak (the
-dominant kernel multiplies in 64-bit fixed point on the integer pipe, so that peak is a yardstick, not
+dominant kernel factors in 64-bit fixed point on the integer pipe, so that peak is a yardstick, not
 its bound); `cpu_baseline` times the CPU restatement of BLAST's algorithm on this host.
 The keys `gemm24`, `lu_ragged`, `mixed_ir` and `adjoint` carry the other workloads (24x24 gemm
 batch, ragged LU, mixed precision + refinement, differentiable solve), each with its timing,

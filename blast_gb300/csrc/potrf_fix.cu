@@ -7,7 +7,7 @@
 // 2,048 matrices with n uniform in 64 .. 512, factored and solved with one right-hand side). In fixed point,
 // with the matrix's rows scaled, the products of earlier columns run on the integer pipe (n <= 128) or on the
 // tensor cores (above), which took the same batch to 9.3 ms and, for its n > 128, to 7.6 ms; binary64 is left
-// with one conversion per factor entry. At n = 512 with three CTAs an SM, three quarters of a CTA's time are
+// with one conversion per factor entry, and with what cannot be certified. At n = 512 with three CTAs an SM, three quarters of a CTA's time are
 // the products (tensor pipe 63% busy meanwhile, the rest taking entries apart into digits and waiting for
 // the staged columns), 8% the diagonal blocks, 8% the rows below them, 7% the conversion. At n = 128
 // the products are half, the diagonal blocks' chains a quarter.
@@ -22,7 +22,7 @@
 //    eight.
 //  * The first chunk's first 32 rows: one warp, a row per lane, the 16 columns right-looking in
 //    registers, the pivot row's limbs by shuffles. The reciprocal square root is integer as well.
-//  * Other rows: a row per thread against the diagonal block, left-looking in registers.
+//  * Other rows: a row per thread against the diagonal block, right-looking in registers.
 //  * A row of a panel that cannot be certified (fix64.cuh) is not stored. After its chunk the columns so far
 //    become binary64, and what is left of the matrix is factored in binary64 (potrf_strips.cuh).
 //  * The factor stays in fixed point in the workspace (L itself, unless the caller says otherwise), as
@@ -59,6 +59,8 @@ struct Shape {
     static constexpr int kScale = kRsqrt + kNB * 16;
     static constexpr int kRow = kScale + NMAX * 2;
     static constexpr int kBytes = kRow + NMAX * 4;
+    // solve_row reads past the diagonal block's last row: rows up to 18.
+    static_assert(kDiag + 8 * (18 * kNB + kNB) <= kBytes);
 };
 
 template <int T>

@@ -18,8 +18,9 @@ as BLAST's do. Three transports:
 
 Device buffers are allocated once per pipeline and reused.
 
-L and X agree with a solve of the same batch in device memory to rounding, not always to the bit: for 17 <= n <= 64
-the kernel, and with it the rounding, follows from the size of the batch that one launch gets (a chunk here).
+L and X agree with a solve of the same batch in device memory to rounding, not always to the bit: the kernel, and with
+it the rounding, follows from the size of the batch that one launch gets (a chunk here) and from the transport, and above
+n = 64 the mirror transport solves on threads where the device call uses CTAs.
 """
 from __future__ import annotations
 

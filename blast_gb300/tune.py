@@ -18,6 +18,8 @@ Tunable choices (read by the library through blastgpu_tune_set / tune_get_bin):
   this module: from 65 on the library weighs batch and right-hand sides).
 * ``posv.warp.n<bin>`` — ragged binary64 Cholesky solves with every n <= 128: the substitutions (and
   for n <= 16 the factor) by one warp (1) or one CTA (0) per matrix (within 10 n eps of each other).
+* ``potrf_fix.threads.n<bin>`` — threads of the CTA that factors a matrix in fixed point (32 up to n = 64, 64 up to 128,
+  else 128; same factor; not timed by this module).
 * ``posv.quad.n<bin>`` — uniform Cholesky batches that run in binary64 on a thread per matrix run a
   quad of lanes per matrix when they hold fewer than value / 100 full warps per SM sub-partition (same bits; not
   timed by this module: the library's defaults, 0 / 50 / 150 / 150 / 150 / 150 for the bins 8 to

@@ -27,8 +27,9 @@
  * Results agree with BLAST's algorithm run on the same inputs to a normwise relative error <=
  * 10*n*eps. Most kernels reproduce BLAST's order of IEEE binary64 fused multiply-adds exactly; Cholesky
  * divides by a pivot as a multiplication by its reciprocal, and from n = 17 on factors square matrices in
- * 64-bit fixed point scaled row by row (entries held to 2^-60 of their row's norm), save large uniform
- * batches of sizes that one binary64 thread per matrix does sooner.
+ * 64-bit fixed point scaled row by row, save uniform batches that one binary64 thread per matrix does sooner. What
+ * fixed point cannot serve (weakly coupled unknowns, tiny or no pivots, non-finite entries) is factored in
+ * binary64, from the panel on where that shows, so that info and NaN are binary64's; all solves are binary64.
  */
 #ifndef BLASTGPU_H
 #define BLASTGPU_H
@@ -105,7 +106,9 @@ int blastgpu_probe_mma_tflops(int kind, double* tflops, blastgpu_stream_t stream
  * buffers; on hardware-coherent systems such as GB300 any host allocation), so a host-resident batch
  * is solved without staging copies. Up to n = 64 the working copies are shared memory as a rule;
  * otherwise the factorisation re-reads its partial results from the device workspaces L_work (n*n
- * doubles per instance) and X_work (n*nrhs per instance), which must be device memory. Same results as blastgpu_dposv_strided, bit for bit.
+ * doubles per instance) and X_work (n*nrhs per instance), which must be device memory. Up to n = 64 the same bits as
+ * blastgpu_dposv_strided where both take the same kernel (batches in host memory choose by rules of their own);
+ * otherwise the same to rounding.
  * No reference counterpart (BLAST's matrices are host memory by construction). */
 int blastgpu_dposv_mirror_strided(int n, int nrhs, const double* A, int lda, int64_t stride_a,
                                   const double* B, int ldb, int64_t stride_b, double* L, int ldl,
@@ -256,7 +259,7 @@ int blastgpu_dpotrf_batched(const blastgpu_potrf_desc* desc, int64_t batch, int 
                             int32_t* info, blastgpu_stream_t stream);
 
 /* potrf followed by the two triangular solves L*Y = B, L^T*X = Y (BLAST has no potrs; this is
- * potrf + trsm<Lower> + trsm<Upper> on trans(L), dense/Trsm.hpp:17-66), fused in one kernel.
+ * potrf + trsm<Lower> + trsm<Upper> on trans(L), dense/Trsm.hpp:17-66), in one kernel up to n = 64.
  * B is n x nrhs; X may equal B; L may equal A. */
 int blastgpu_dposv_strided(int n, int nrhs, const double* A, int lda, int64_t stride_a,
                            double* L, int ldl, int64_t stride_l,
