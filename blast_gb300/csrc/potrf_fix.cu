@@ -396,15 +396,20 @@ struct RowState {
     int any = 0;
 };
 
-// Whether row i is certified; its word after the panel. One thread. Out of line, and as few instructions as can be:
-// what is executed once in a while is not in the instruction cache (n = 128 x 4,000, with five weak entries a
-// matrix: 1.72 ms, 2.05 when a row with one was gone through entry by entry, 1.51 without a look at them).
+// Row i's word after the panel.
+__device__ __forceinline__ void note_row(Panel const& p, int i, RowState const& s) {
+    p.row[i] = fix64::row_after(p.row[i], p.k0 / kNB, s.squares, s.any != 0);
+}
+
+// Whether row i is certified, once its word and the diagonal block's rows' are noted. One thread. Out of line, and as
+// few instructions as can be: what is executed once in a while is not in the instruction cache (n = 128 x 4,000, with
+// five weak entries a matrix: 1.72 ms, 2.05 when a row with one was gone through entry by entry, 1.51 without a look
+// at them).
 template <int T>
-__device__ __noinline__ bool certified(Panel const p, int i, const int64_t* x, RowState const s) {
-    uint32_t const now = fix64::row_after(p.row[i], p.k0 / kNB, s.squares, s.any != 0);
-    p.row[i] = now;
-    return s.ok && (now & fix64::kTodo) == 0 && (now & fix64::kNormMask) <= fix64::kNormMost &&
-           (s.weak == 0 || served<T>(p, i, x, s.weak));
+__device__ __noinline__ bool certified(Panel const p, int i, const int64_t* x, bool in_range, unsigned weak) {
+    uint32_t const word = p.row[i];
+    return in_range && (word & fix64::kTodo) == 0 && (word & fix64::kNormMask) <= fix64::kNormMost &&
+           (weak == 0 || served<T>(p, i, x, weak));
 }
 
 // Row i of the panel to the workspace, its first `entries` columns, if it is certified; else it is left to binary64.
@@ -467,9 +472,10 @@ __device__ __forceinline__ void factor_diagonal(Panel const& p, int mr, int64_t*
             if (u == 1) pivot(c);
         }
     });
+    if (mine) note_row(p, lane, state);
     __syncwarp();
     // The diagonal block's rows are certified before any row is stored.
-    bool const ok = mine && certified<T>(p, lane, C + lane, state);
+    bool const ok = mine && certified<T>(p, lane, C + lane, state.ok, state.weak);
     if (__all_sync(0xffffffffu, good && (ok || !mine || lane >= nb))) {
         if (mine) store_row<T>(p, lane, min(lane + 1, nb), C + lane, ok);
     } else if (lane == 0) {
@@ -501,7 +507,8 @@ __device__ __forceinline__ void solve_row(Panel const& p, int i, int r, int64_t*
 #pragma unroll
         for (int u = 1; u < decltype(left)::value; ++u) fix64::take_off(sum, cross, u, v, d[u * kNB]);
     });
-    store_row<T>(p, i, kNB, C + r, certified<T>(p, i, C + r, state));
+    note_row(p, i, state);
+    store_row<T>(p, i, kNB, C + r, certified<T>(p, i, C + r, state.ok, state.weak));
 }
 
 // One matrix. W: the fixed-point factor while the matrix is being factored, n rows of 8 bytes per
