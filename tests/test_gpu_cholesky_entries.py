@@ -250,3 +250,34 @@ def test_info_is_binary64s(gpu, oracle_lib, n):
         assert info[k] == want, (k, int(info[k]), want)
         if want == 0:
             assert np.allclose(np.tril(got[k]), np.tril(ref), rtol=10 * n * EPS, atol=0)
+
+
+def structured(rng, n):
+    """A sparse graph with weights over 12 decades, a Gram matrix with entries over 8, blocks with a weak dense coupling, a
+    kernel in random order, and a matrix with one tiny entry among others that are not."""
+    M = np.triu(rng.random((n, n)) < 0.2, 1) * 10.0 ** rng.uniform(-12, 0, (n, n)) * rng.choice([-1, 1], (n, n))
+    M = M + M.T
+    yield M + np.diag(np.abs(M).sum(1) * rng.uniform(1, 2) + 10.0 ** rng.uniform(-3, 0, n))
+    G = rng.standard_normal((n, n)) * 10.0 ** rng.uniform(-8, 0, (n, n)) * (rng.random((n, n)) < 0.5)
+    yield G @ G.T + 10.0 ** rng.uniform(-4, 0) * np.eye(n)
+    A, h = np.zeros((n, n)), n // 3
+    A[:h, :h], A[h:, h:] = spd(rng, h), spd(rng, n - h)
+    C = rng.standard_normal((n, n)) * 10.0 ** rng.uniform(-14, -1)
+    yield A + 0.05 * (C + C.T)
+    x = rng.uniform(0, rng.choice([3, 10, 30]), n)
+    yield np.exp(-np.abs(x[:, None] - x) ** 1.5) + 10.0 ** rng.uniform(-3, 0) * np.eye(n)
+    A = spd(rng, n)
+    A[n - 1, 1] = A[1, n - 1] = 10.0 ** rng.uniform(-20, -3)
+    yield A
+
+
+@pytest.mark.parametrize("n", [17, 48, 64, 100])
+def test_structured_matrices(gpu, n):
+    """Every entry of the solution, whatever becomes of single small entries of the factor."""
+    rng = np.random.default_rng(n)
+    As = [A for _ in range(12) for A in structured(rng, n)]
+    Bs = [np.stack([np.eye(n)[rng.integers(n)], rng.standard_normal(n)], 1) for _ in As]
+    info, _, X = run(gpu, As, Bs)
+    assert not info.any()
+    for A, B, x in zip(As, Bs, X):
+        check(A, B, x)
